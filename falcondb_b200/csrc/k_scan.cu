@@ -14,6 +14,7 @@
 #include "common.cuh"
 #include "engine.h"
 #include "stream.cuh"
+#include "where.cuh"
 
 namespace fdb {
 
@@ -101,21 +102,22 @@ __device__ double i128_to_f64(uint64_t lo, int64_t hi) {
   return (double)hi * 18446744073709551616.0 + (double)lo;
 }
 
+// Tile rows per column and ring depth: ~64 KB of staging per CTA so that three
+// CTAs (24 consumer warps) fit on one SM.
+template <int NC>
+struct TileShape {
+  static constexpr int TR = NC == 1 ? 2048 : 1024;
+  static constexpr int STAGES = NC <= 2 ? 4 : 3;
+  static constexpr int NCW = 8;
+};
 struct ScanAggParams {
   PredProg prog;
   ScanCols sc;
   int32_t naggs;
   int32_t func[4];
   int32_t acol[4];
-  // FilterAggOp's decoded WHERE: one compare of column f_cmp_col (-1: none)
-  // against a literal, as double (f_cmp_f64) or as int64; f_cmp_mask holds
-  // the accepted outcomes (bit 0 unordered, 1 less, 2 equal, 3 greater).
-  int32_t f_cmp_col;
-  uint32_t f_cmp_mask;
-  int32_t f_cmp_f64;
+  WhereProg where;        // FilterAggOp: the same program, decoded
   uint32_t f_agg_f64;     // bit a: aggregate a's column is FLOAT64
-  double f_lit_f;
-  int64_t f_lit_i;
   AggAcc* partials;       // [gridDim.x * 4]
   unsigned int* ticket;   // zero on entry; reset by the last CTA
   fdb_agg_value* out;     // [naggs] or nullptr
@@ -303,15 +305,14 @@ __device__ __forceinline__ void fold_value(AggAcc& a, int f, T v) {
   a.n++;
 }
 
-// Aggregates with at most one `col op literal` WHERE, every column NULL-free
-// and numeric (SELECT SUM(score), AVG(salary) ... WHERE score > 50).  A thread
-// takes its rows of the tile four at a time (ctid, ctid + nct, ...): it
-// compares them into a 4-bit mask, branch-free, and then each aggregate folds
-// the four rows under the mask with selects, not branches, so the aggregate
-// function and the column type are decided once per four rows (a uniform
-// branch), not per row as ScanAggOp's interpreter does.  Groups of four rows
-// that lie wholly inside the tile (all but at most one per tile) load without
-// bounds checks.
+// Aggregates under any WHERE program, over nullable or NULL-free columns.  A
+// thread takes its rows of the tile four at a time (ctid, ctid + nct, ...): the
+// program gives a 4-bit mask of the rows that pass (where_mask), a nullable
+// column's validity another, and then each aggregate folds the four rows under
+// its mask with selects, not branches, so the aggregate function and the column
+// type are decided once per four rows (a uniform branch), not per row as
+// ScanAggOp's interpreter does.  Groups of four rows that lie wholly inside the
+// tile (all but at most one per tile) load without bounds checks.
 //
 // While rows are folded, two accumulators hold other forms than ScanAggOp's,
 // which finish() converts back before the shared partials / final pass:
@@ -323,11 +324,14 @@ __device__ __forceinline__ void fold_value(AggAcc& a, int f, T v) {
 //     first row) and compares doubles: NaN compares false and never takes
 //     part (f64::min / max), and on equal values the sign bits are combined
 //     so that +0.0 wins a MAX and -0.0 a MIN, as their order keys do.
-// FilterAggOp's launch shape: 2048-row tiles, two stages, and registers held
-// to three resident CTAs per SM (72, no spills).  On COUNT, SUM(score),
-// AVG(salary), MAX(score) WHERE score > 50 over 100M rows this took the query
-// from 0.443 ms (1024-row tiles, four stages, two CTAs per SM) to 0.362 ms;
-// 2048 x 3 stages: 0.386; 1024 x 3 stages at 3 CTAs: 0.390.
+// FilterAggOp's launch shape: 2048-row tiles (1024 with three or four columns,
+// so that three CTAs' rings still fit an SM), two stages, and registers held to
+// three resident CTAs per SM (72, no spills).  Bound by instruction issue and
+// by latency at 24 consumer warps per SM, not by HBM.  COUNT, SUM(score),
+// AVG(salary), MAX(score): WHERE score > 50 over 100M rows 0.318 ms (0.362 with
+// a one-compare form that tested four outcomes per row and selected around
+// every MAX); WHERE score > 50 AND salary < 150000 over 33.3M rows with NULL
+// scores 0.176 ms, where ScanAggOp takes 0.791 ms.
 #ifndef FDB_FA_TR
 #define FDB_FA_TR 2048
 #endif
@@ -355,63 +359,21 @@ struct FilterAggOp : ScanAggOp {
       if (a < p.naggs && f64_minmax(p, a)) st.a[a].f = p.func[a] == FDB_AGG_MIN ? inf : -inf;
   }
 
-  template <bool kFull, typename T, class Acc>
-  static __device__ __forceinline__ void load_r(T (&x)[R], const Acc& acc, int col, const uint32_t (&i)[R],
-                                                uint32_t ok) {
-#pragma unroll
-    for (int j = 0; j < R; ++j)
-      x[j] = (kFull || ((ok >> j) & 1u)) ? acc.template get<T>(col, i[j]) : T(0);
-  }
-
-  template <bool kFull, class Acc>
-  static __device__ __forceinline__ uint32_t pass_mask(const Params& p, const Acc& acc, const uint32_t (&i)[R],
-                                                       uint32_t ok) {
-    const int pc = p.f_cmp_col;
-    if (pc < 0) return ok;
-    const uint32_t amask = p.f_cmp_mask;
-    const bool a_un = amask & 1u, a_lt = (amask >> 1) & 1u, a_eq = (amask >> 2) & 1u, a_gt = (amask >> 3) & 1u;
-    uint32_t m = 0;
-    if (p.f_cmp_f64) {
-      const double lit = p.f_lit_f;
-      const bool lit_nan = lit != lit;  // every outcome is then unordered
-      double x[R];
-      if (p.sc.cols[pc].dtype == FDB_FLOAT64) {
-        load_r<kFull, double>(x, acc, pc, i, ok);
-      } else {
-        int64_t y[R];
-        load_r<kFull, int64_t>(y, acc, pc, i, ok);
-#pragma unroll
-        for (int j = 0; j < R; ++j) x[j] = (double)y[j];
-      }
-#pragma unroll
-      for (int j = 0; j < R; ++j) {
-        const bool pass = (a_lt && x[j] < lit) || (a_eq && x[j] == lit) || (a_gt && x[j] > lit) ||
-                          (a_un && (lit_nan || x[j] != x[j]));
-        m |= (pass ? 1u : 0u) << j;
-      }
-    } else {
-      const int64_t lit = p.f_lit_i;
-      int64_t x[R];
-      load_r<kFull, int64_t>(x, acc, pc, i, ok);
-#pragma unroll
-      for (int j = 0; j < R; ++j) {
-        const bool pass = (a_lt && x[j] < lit) || (a_eq && x[j] == lit) || (a_gt && x[j] > lit);
-        m |= (pass ? 1u : 0u) << j;
-      }
-    }
-    return kFull ? m : m & ok;
+  static __device__ __forceinline__ void prefetch(const Params& p, uint64_t row0, uint32_t rows) {
+    prefetch_valid(p.where.nullable, p.sc.cols, row0, rows);
   }
 
   template <bool kFull, typename T, class Acc>
   static __device__ __forceinline__ void fold_r(AggAcc& a, int f, const Acc& acc, int col, const uint32_t (&i)[R],
                                                 uint32_t ok, uint32_t m) {
     T x[R];
-    load_r<kFull, T>(x, acc, col, i, ok);
+    where_load<kFull, R>(x, acc, col, i, ok);
     if (f == FDB_AGG_SUM || f == FDB_AGG_AVG) {
       if constexpr (T(0.5) != T(0)) {
         double s = 0.0;
 #pragma unroll
-        for (int j = 0; j < R; ++j) s += ((m >> j) & 1u) ? x[j] : 0.0;
+        for (int j = 0; j < R; ++j)
+          if ((m >> j) & 1u) s += x[j];
         a.f += s;
       } else {
         uint64_t lo = 0;
@@ -429,18 +391,28 @@ struct FilterAggOp : ScanAggOp {
       return;
     }
     if constexpr (T(0.5) != T(0)) {
+      // A value that reaches the running extreme is rare after a thread's first
+      // rows: one compare per row finds it, and only then is it looked at.
       const bool is_max = f == FDB_AGG_MAX;
+      uint32_t num = 0, reach = 0;
 #pragma unroll
       for (int j = 0; j < R; ++j) {
-        const bool in = (m >> j) & 1u;
-        const double v = x[j];
-        if (in && (is_max ? v > a.f : v < a.f)) {
-          a.f = v;
-        } else if (in && v == a.f) {
-          const uint64_t fb = (uint64_t)__double_as_longlong(a.f), vb = (uint64_t)__double_as_longlong(v);
-          a.f = __longlong_as_double((long long)(is_max ? (fb & vb) : (fb | vb)));
+        num |= (x[j] == x[j] ? 1u : 0u) << j;
+        reach |= ((is_max ? x[j] >= a.f : x[j] <= a.f) ? 1u : 0u) << j;
+      }
+      a.n += (uint64_t)__popc(m & num);
+      if (reach & m) {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          if (!((reach & m) >> j & 1u)) continue;
+          const double v = x[j];
+          if (is_max ? v > a.f : v < a.f) {
+            a.f = v;
+          } else if (v == a.f) {
+            const uint64_t fb = (uint64_t)__double_as_longlong(a.f), vb = (uint64_t)__double_as_longlong(v);
+            a.f = __longlong_as_double((long long)(is_max ? (fb & vb) : (fb | vb)));
+          }
         }
-        a.n += (in && v == v) ? 1u : 0u;
       }
     } else {
 #pragma unroll
@@ -456,22 +428,28 @@ struct FilterAggOp : ScanAggOp {
     }
   }
 
-  template <bool kFull, class Acc>
+  template <bool kFull, int kStride, class Acc>
   static __device__ __forceinline__ void group(Local& st, const Params& p, const Acc& acc, uint32_t b,
-                                               uint32_t rows, int ctid, int nct) {
+                                               uint32_t rows, int ctid) {
     uint32_t i[R];
     uint32_t ok = 0;
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      i[j] = b + (uint32_t)j * (uint32_t)nct + (uint32_t)ctid;
+      i[j] = b + (uint32_t)j * kStride + (uint32_t)ctid;
       ok |= (kFull || i[j] < rows ? 1u : 0u) << j;
     }
-    const uint32_t m = pass_mask<kFull>(p, acc, i, ok);
+    const uint32_t valid = valid_masks<kFull, R, kStride>(p.where.nullable, p.sc.cols, acc, i, ok);
+    const uint32_t pass = where_mask<kFull, R>(p.where, acc, p.sc.cols, i, ok, valid);
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
       if (a >= p.naggs) break;
       const int f = p.func[a];
-      if (f == FDB_AGG_COUNT_STAR || f == FDB_AGG_COUNT)
+      if (f == FDB_AGG_COUNT_STAR) {
+        st.a[a].n += (uint64_t)__popc(pass);
+        continue;
+      }
+      const uint32_t m = pass & (valid >> (p.acol[a] * R));
+      if (f == FDB_AGG_COUNT)
         st.a[a].n += (uint64_t)__popc(m);
       else if ((p.f_agg_f64 >> a) & 1u)
         fold_r<kFull, double>(st.a[a], f, acc, p.acol[a], i, ok, m);
@@ -483,10 +461,11 @@ struct FilterAggOp : ScanAggOp {
   template <class Acc>
   static __device__ void step(Local& st, const Params& p, unsigned char*, const Acc& acc, uint32_t rows, int ctid,
                               int nct) {
-    const uint32_t g = R * (uint32_t)nct;
+    constexpr int kStride = TileShape<1>::NCW * 32;  // the consumer threads of every launch
+    const uint32_t g = R * kStride;
     uint32_t b = 0;
-    for (; b + g <= rows; b += g) group<true>(st, p, acc, b, rows, ctid, nct);
-    if (b < rows) group<false>(st, p, acc, b, rows, ctid, nct);
+    for (; b + g <= rows; b += g) group<true, kStride>(st, p, acc, b, rows, ctid);
+    if (b < rows) group<false, kStride>(st, p, acc, b, rows, ctid);
   }
 
   // Back to ScanAggOp's accumulator forms, then its reduction and final pass.
@@ -677,14 +656,6 @@ struct DistinctOp {
 // ---------------------------------------------------------------------------
 // Launch helpers for the streamer.
 // ---------------------------------------------------------------------------
-// Tile rows per column and ring depth: ~64 KB of staging per CTA so that three
-// CTAs (24 consumer warps) fit on one SM.
-template <int NC>
-struct TileShape {
-  static constexpr int TR = NC == 1 ? 2048 : 1024;
-  static constexpr int STAGES = NC <= 2 ? 4 : 3;
-  static constexpr int NCW = 8;
-};
 template <int NC, int TRo, int STo = 0>
 struct TileShapeO {
   static constexpr int TR = TRo ? TRo : TileShape<NC>::TR;
@@ -733,6 +704,23 @@ static void launch_stream_nc(Ctx& c, const fdb_dev_column* cols, int ncols, uint
     case 3: launch_stream<Op, 3, TRo, 8, STo, MINB>(c, cols, n, p, op_smem); break;
     case 4: launch_stream<Op, 4, TRo, 8, STo, MINB>(c, cols, n, p, op_smem); break;
     default: fail(FDB_E_ARG, "between 1 and 4 input columns are supported per scan");
+  }
+}
+
+// FilterAggOp over p's program and aggregates.  Its split INT64 sums are exact
+// below 2^32 rows per thread, so from 2^40 rows on the interpreter takes over.
+static void launch_filter_agg(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n, ScanAggParams& p) {
+  if (n >= (1ull << 40)) {
+    launch_stream_nc<ScanAggOp>(c, cols, ncols, n, p, ScanAggOp::kSmem);
+    return;
+  }
+  fill_where(p.where, p.prog, p.sc.cols, ncols);
+  constexpr int kTr = FDB_FA_TR, kSt = FDB_FA_STAGES, kMin = FDB_FA_MINB;
+  switch (ncols) {
+    case 1: launch_stream<FilterAggOp, 1, kTr, 8, kSt, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
+    case 2: launch_stream<FilterAggOp, 2, kTr, 8, kSt, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
+    case 3: launch_stream<FilterAggOp, 3, kTr / 2, 8, kSt, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
+    default: launch_stream<FilterAggOp, 4, kTr / 2, 8, kSt, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
   }
 }
 
@@ -812,29 +800,9 @@ void op_aggregate(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,
       launch_stream<ColAggOp<int64_t>, 1>(c, cols, n, p, ScanAggOp::kSmem);
     return;
   }
-  // At most one `col op literal` and NULL-free numeric columns: FilterAggOp
-  // (whose split INT64 sums are exact below 2^32 rows per thread).
-  bool fast = (nterms == 0 || (nterms == 1 && prog[0].kind == FDB_TERM_CMP)) && n < (1ull << 40);
-  for (int i = 0; i < ncols && fast; ++i) fast = cols[i].validity == nullptr && cols[i].dtype != FDB_UTF8;
-  if (fast) {
-    p.f_cmp_col = -1;
-    if (nterms == 1) {
-      const fdb_pred_term& t = prog[0];
-      p.f_cmp_col = t.col;
-      // Accepted outcomes of x op lit (bit 0 unordered, 1 less, 2 equal, 3
-      // greater): NaN passes != only, as cmp_op does.
-      static const uint32_t kAccept[6] = {0x4u, 0xBu, 0x2u, 0x6u, 0x8u, 0xCu};
-      p.f_cmp_mask = kAccept[t.op];
-      p.f_cmp_f64 = cols[t.col].dtype == FDB_FLOAT64 || t.lit_type == FDB_FLOAT64;
-      p.f_lit_f = t.lit_type == FDB_FLOAT64 ? t.lit_f : (double)t.lit_i;
-      p.f_lit_i = t.lit_i;
-    }
-    for (int a = 0; a < naggs; ++a)
-      if (aggs[a].func != FDB_AGG_COUNT_STAR && cols[aggs[a].col].dtype == FDB_FLOAT64) p.f_agg_f64 |= 1u << a;
-    launch_stream_nc<FilterAggOp, FDB_FA_TR, FDB_FA_STAGES, FDB_FA_MINB>(c, cols, ncols, n, p, ScanAggOp::kSmem);
-    return;
-  }
-  launch_stream_nc<ScanAggOp>(c, cols, ncols, n, p, ScanAggOp::kSmem);
+  for (int a = 0; a < naggs; ++a)
+    if (aggs[a].func != FDB_AGG_COUNT_STAR && cols[aggs[a].col].dtype == FDB_FLOAT64) p.f_agg_f64 |= 1u << a;
+  launch_filter_agg(c, cols, ncols, n, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -950,7 +918,7 @@ void op_filter_count(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,
       launch_cmp_count<int64_t, int64_t>(c, cols, n, p, prog[0].op);
     return;
   }
-  launch_stream_nc<ScanAggOp>(c, cols, ncols, n, p, ScanAggOp::kSmem);
+  launch_filter_agg(c, cols, ncols, n, p);
 }
 
 void op_distinct_codes(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,
@@ -975,41 +943,61 @@ void op_distinct_codes(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n
 }
 
 // ---------------------------------------------------------------------------
-// WHERE mask: one warp per 64-row word, two ballots per word; padding bits zero.
+// WHERE mask: one ballot per 32 rows; padding bits zero.
 // ---------------------------------------------------------------------------
 struct MaskParams {
-  PredProg prog;
+  WhereProg where;
   ScanCols sc;
 };
 
-__device__ __forceinline__ bool row_passes(const MaskParams& p, uint64_t row) {
-  auto get = [&](int c, int64_t& iv, double& fv, uint32_t& code, bool& valid) -> int {
-    const DevCol& col = p.sc.cols[c];
-    const int dt = col.dtype;
-    if (dt == FDB_FLOAT64)
-      fv = static_cast<const double*>(col.values)[row];
-    else if (dt == FDB_INT64)
-      iv = static_cast<const int64_t*>(col.values)[row];
-    else
-      code = static_cast<const uint32_t*>(col.values)[row];
-    valid = col.validity ? col_valid(col, row) : true;
-    return dt;
-  };
-  return eval_prog(p.prog, get);
-}
+// A warp's rows row0 + j * 32 + lane, read straight from the columns: a
+// compare reads eight values per thread, all in flight together.
+struct MaskAcc {
+  const ScanCols& sc;
+  uint64_t row0;
+  template <typename T>
+  __device__ __forceinline__ T get(int c, uint32_t i) const {
+    return __ldcs(static_cast<const T*>(sc.cols[c].values) + row0 + i);
+  }
+  __device__ __forceinline__ uint64_t row(uint32_t i) const { return row0 + i; }
+};
 
-__global__ void filter_mask_kernel(MaskParams p, uint64_t n, uint64_t* mask) {
+// Bound by HBM: a warp takes 256 rows (four mask words) per step, so a compare
+// has eight loads per thread in flight.  Two compares over 40M rows (0.64 GB):
+// 0.098 ms, against 0.282 ms with the row-by-row interpreter.
+constexpr int kMaskRows = 8;
+__global__ void __launch_bounds__(256) filter_mask_kernel(const __grid_constant__ MaskParams p, uint64_t n,
+                                                          uint64_t* mask) {
+  constexpr int R = kMaskRows;
   const uint64_t nwords = (n + 63) / 64;
   const int lane = threadIdx.x & 31;
   const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t w = gw; w < nwords; w += nwarps) {
-    const uint64_t r0 = w * 64 + lane, r1 = r0 + 32;
-    const bool a = r0 < n && row_passes(p, r0);
-    const bool b = r1 < n && row_passes(p, r1);
-    const uint32_t lo = __ballot_sync(0xffffffffu, a);
-    const uint32_t hi = __ballot_sync(0xffffffffu, b);
-    if (lane == 0) mask[w] = (uint64_t)lo | ((uint64_t)hi << 32);
+  uint32_t i[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) i[j] = j * 32 + lane;
+  for (uint64_t g = gw; g * (R * 32) < n; g += nwarps) {
+    const MaskAcc acc{p.sc, g * (R * 32)};
+    const uint64_t left = n - acc.row0;
+    uint32_t m;
+    if (left >= R * 32) {
+      const uint32_t v = valid_masks<true, R, 32>(p.where.nullable, p.sc.cols, acc, i, 0xFFu);
+      m = where_mask<true, R>(p.where, acc, p.sc.cols, i, 0xFFu, v);
+    } else {
+      uint32_t ok = 0;
+#pragma unroll
+      for (int j = 0; j < R; ++j) ok |= (i[j] < left ? 1u : 0u) << j;
+      const uint32_t v = valid_masks<false, R, 32>(p.where.nullable, p.sc.cols, acc, i, ok);
+      m = where_mask<false, R>(p.where, acc, p.sc.cols, i, ok, v);
+    }
+    uint32_t half = 0;  // lane j keeps half word j
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const uint32_t b = __ballot_sync(0xffffffffu, (m >> j) & 1u);
+      if (lane == j) half = b;
+    }
+    const uint64_t w32 = g * R + lane;
+    if (lane < R && w32 < nwords * 2) reinterpret_cast<uint32_t*>(mask)[w32] = half;
   }
 }
 
@@ -1018,11 +1006,13 @@ void op_filter_mask(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,
   MaskParams p;
   std::memset(&p, 0, sizeof(p));
   fill_cols(p.sc, cols, ncols, n);
-  fill_prog(p.prog, prog, nterms, ncols);
+  PredProg pp;
+  fill_prog(pp, prog, nterms, ncols);
+  fill_where(p.where, pp, p.sc.cols, ncols);
   const uint64_t nwords = (n + 63) / 64;
   if (nwords == 0) return;
   const int threads = 256;
-  const uint64_t blocks = umin64((nwords + 7) / 8, (uint64_t)c.sm_count * 8);
+  const uint64_t blocks = umin64((nwords + 31) / 32, (uint64_t)c.sm_count * 8);
   filter_mask_kernel<<<(unsigned)blocks, threads, 0, c.stream>>>(p, n, d_mask);
   FDB_CUDA(cudaGetLastError());
 }

@@ -12,6 +12,8 @@
 // grid-stride loop.  Every wait is bounded (kSpinLimit); on time-out the kernel
 // records kErrTimeout in the context's error word and winds down.
 #pragma once
+#include <utility>
+
 #include "common.cuh"
 
 namespace fdb {
@@ -108,12 +110,28 @@ inline uint64_t stream_m_end(const void* const* bases, int nc, uint64_t n) {
 //   static __device__ void finish(Local&, const Params&, unsigned char* op_smem, int ctid, int nct);
 // step() and finish() are executed by all consumer threads; block-wide syncs
 // inside them must use consumer_bar(nct).
+// An op may also have
+//   static __device__ void prefetch(const Params&, uint64_t row0, uint32_t rows);
+// run by the producer lane when it stages rows [row0, row0 + rows), a ring's
+// depth before step() sees them: what step() reads besides the staged columns
+// (validity words) can be brought into L2 there.
 // MINB: resident CTAs per SM the register allocation must allow (0: none).
 // DYN: tiles are handed out by an atomic counter (src.tile_ctr) instead of
 // round-robin, so CTAs that run faster take more tiles and all finish
 // together.  The tile order then varies run to run, so DYN is only for ops
 // whose result does not depend on it (top-k, counts), and for ops whose step
 // has no CTA-wide barrier: on a time-out a warp leaves the tile loop at once.
+template <class Op, class = void>
+struct OpPrefetch {
+  static __device__ __forceinline__ void run(const typename Op::Params&, uint64_t, uint32_t) {}
+};
+template <class Op>
+struct OpPrefetch<Op, decltype(Op::prefetch(std::declval<const typename Op::Params&>(), uint64_t(), uint32_t()))> {
+  static __device__ __forceinline__ void run(const typename Op::Params& p, uint64_t row0, uint32_t rows) {
+    Op::prefetch(p, row0, rows);
+  }
+};
+
 template <class Op, int NC, int TR, int STAGES, int NCW, int CB = 8, int MINB = 1, bool DYN = false>
 __global__ void __launch_bounds__((NCW + 1) * 32, MINB)
     stream_kernel(StreamSrc<NC> src, typename Op::Params p, int* err, int op_smem_off) {
@@ -171,6 +189,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, MINB)
         for (int c = 0; c < NC; ++c)
           bulk_g2s(tiles + ((size_t)s * NC + c) * TR * CB, src.base[c] + r0 * src.esize[c],
                    rows * src.esize[c], &full[s], policy);
+        OpPrefetch<Op>::run(p, r0, rows);
       }
     }
     return;  // consumers sync among themselves with named barrier 1
