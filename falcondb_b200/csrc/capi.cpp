@@ -108,6 +108,23 @@ void Ctx::ensure_scratch(size_t bytes) {
   scratch = alloc_buf(want);
 }
 
+bool Ctx::try_scratch(size_t bytes) {
+  if (scratch.bytes >= bytes) return true;
+  const size_t want = (bytes + (1u << 20) - 1) & ~size_t((1u << 20) - 1);
+  const size_t others = in_use.load() - scratch.bytes;
+  if (others >= budget || want > (budget - others) / 4) return false;
+  void* p = nullptr;
+  if (cudaMallocAsync(&p, want, stream) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (scratch.ptr) free_buf(scratch);
+  scratch.ptr = p;
+  scratch.bytes = want;
+  in_use += want;
+  return true;
+}
+
 void* Ctx::scratch_take(size_t bytes) {
   const size_t aligned = (bytes + 255) & ~size_t(255);
   if (scratch_top + aligned > scratch.bytes)

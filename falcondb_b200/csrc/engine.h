@@ -110,6 +110,10 @@ struct Ctx {
   void* scratch_take(size_t bytes);
   void scratch_reset() { scratch_top = kTicketBytes; }
   void ensure_scratch(size_t bytes);
+  // ensure_scratch for a working buffer that an operator can do without: false,
+  // and nothing changes, when it would take more than a quarter of what the
+  // budget has left or the device has no room for it.
+  bool try_scratch(size_t bytes);
   int check_device_error();                      // reads and clears d_err (syncs)
 };
 
