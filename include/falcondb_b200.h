@@ -507,7 +507,7 @@ typedef struct fdb_gb_query {
 } fdb_gb_query;
 
 /* Launch shape and table sizing of a batch; zero fields take defaults
- * (load factor 0.5, 2 CTAs per SM, 8192-row tiles). */
+ * (load factor 0.5, 3 CTAs per SM, 8192-row tiles). */
 typedef struct fdb_batch_tuning {
     double  load_factor;       /* table slots = 2 x expected groups / load_factor, pow2 */
     int32_t ctas_per_sm;       /* persistent CTAs per SM (capped by occupancy)    */
