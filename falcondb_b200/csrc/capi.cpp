@@ -654,7 +654,7 @@ int fdb_group_by_i64(fdb_db* db, const fdb_dev_column* key, const fdb_dev_column
     CallScope s(db, default_scratch(c));
     const GbSizing sz = group_by_i64_sizing(s.c, *key, nrows, expected_groups);
     s.c.scratch_reset();
-    s.c.ensure_scratch(group_by_i64_scratch(sz, lf) + (16u << 20));
+    reserve_group_by_i64(s.c, sz, lf, nrows, nterms);
     op_group_by_i64(s.c, *key, *value, nrows, prog, nterms, pred_cols, npred_cols, sz, lf, d_groups, capacity,
                     d_ngroups);
   });

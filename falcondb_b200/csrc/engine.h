@@ -175,13 +175,14 @@ struct GbSizing {
   uint64_t groups = 0;
   bool has_range = false;
   int64_t kmin = 0, kmax = 0;
+  std::vector<uint32_t> parts;  // non-NULL keys per hash partition; empty when not counted
 };
 // `expected_groups` when nonzero (no pass over the keys, no range), else the
 // sizing pass over the key column: estimate plus headroom, and the key range
 // (synchronises).
 GbSizing group_by_i64_sizing(Ctx& c, const fdb_dev_column& key, uint64_t n, uint64_t expected_groups);
-// Scratch bytes op_group_by_i64 takes for `s` at `load_factor`.
-size_t group_by_i64_scratch(const GbSizing& s, double load_factor);
+// Reserves scratch for op_group_by_i64 of n rows (on top of what is taken).
+void reserve_group_by_i64(Ctx& c, const GbSizing& s, double load_factor, uint64_t n, int nterms);
 void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& value, uint64_t n,
                      const fdb_pred_term* prog, int nterms, const fdb_dev_column* pred_cols,
                      int npred, const GbSizing& s, double load_factor,
@@ -217,6 +218,7 @@ struct KeyStats {
   uint64_t distinct = 0;
   bool has_range = false;  // false when every key is NULL (or there are none)
   int64_t kmin = 0, kmax = 0;
+  std::vector<uint32_t> parts;  // non-NULL keys per hash partition (below 2^32 keys)
 };
 KeyStats key_stats_i64(Ctx& c, const fdb_dev_column& key, uint64_t n);
 

@@ -26,6 +26,11 @@ constexpr uint32_t kSmemSlots = 1024;      // CTA table slots (power of two)
 constexpr uint32_t kSmemProbe = FDB_GB_SMEM_PROBE;  // probes before a row spills to global
 constexpr uint32_t kGlobalProbeLimit = 1u << 16;
 
+// Hash partitions of a key (the top bits of mix64 of the stored key).
+constexpr uint32_t kGbParts = 512;
+__device__ __forceinline__ uint32_t gb_partition(uint64_t hash) { return (uint32_t)(hash >> 55); }
+static_assert(kGbParts == 1u << 9, "gb_partition takes nine bits");
+
 __device__ __forceinline__ void gslot_accum(GSlot* s, double v, bool has_v) {
   atomicAdd(&s->count, 1ull);
   if (has_v) {

@@ -3,13 +3,15 @@
 // Gandouet, Meunier, "HyperLogLog: the analysis of a near-optimal cardinality
 // estimation algorithm", 2007; 2^12 registers, standard error about 1.6 %),
 // and in the same pass the smallest and largest non-NULL key (NULL = a clear
-// validity bit, or INT64_MIN, which GROUP BY reads as NULL).  One pass over the
-// keys plus a 16 KB device-to-host copy; synchronises the context stream.
+// validity bit, or INT64_MIN, which GROUP BY reads as NULL), and how many of them
+// fall into each hash partition (gb_partition).  One pass over the keys plus an
+// 18 KB device-to-host copy; synchronises the context stream.
 #include <cmath>
 #include <vector>
 
 #include "common.cuh"
 #include "engine.h"
+#include "gtable.cuh"
 
 namespace fdb {
 
@@ -21,10 +23,10 @@ constexpr int kHllRegs = 1 << kHllBits;
 struct KeyStatsOut {
   unsigned int regs[kHllRegs];
   unsigned long long range[2];
+  unsigned int parts[kGbParts];
 };
 
-__device__ __forceinline__ void hll_add(unsigned int* r, int64_t key) {
-  const uint64_t h = mix64((uint64_t)key ^ (1ull << 63));
+__device__ __forceinline__ void hll_add(unsigned int* r, uint64_t h) {
   const uint32_t idx = (uint32_t)(h >> (64 - kHllBits));
   const uint64_t w = (h << kHllBits) | (1ull << (kHllBits - 1));  // bounds the run of zeros
   atomicMax(&r[idx], (unsigned int)__clzll((long long)w) + 1u);
@@ -37,11 +39,14 @@ __device__ __forceinline__ void hll_add(unsigned int* r, int64_t key) {
 __global__ void __launch_bounds__(256) key_stats_kernel(const int64_t* __restrict__ keys, const uint64_t* validity,
                                                         uint64_t voff, uint64_t n, KeyStatsOut* out) {
   __shared__ unsigned int r[kHllRegs];
+  __shared__ unsigned int parts[kGbParts];
   for (int i = threadIdx.x; i < kHllRegs; i += blockDim.x) r[i] = 0;
+  for (int i = threadIdx.x; i < (int)kGbParts; i += blockDim.x) parts[i] = 0;
   __syncthreads();
   uint64_t lo = ~0ull, hi = 0;
   auto take = [&](int64_t k, uint64_t row) {
-    hll_add(r, k);
+    const uint64_t h = mix64((uint64_t)k ^ (1ull << 63));
+    hll_add(r, h);
     bool valid = k != INT64_MIN;
     if (validity) {
       const uint64_t b = voff + row;
@@ -51,6 +56,7 @@ __global__ void __launch_bounds__(256) key_stats_kernel(const int64_t* __restric
       const uint64_t o = i64_ord_key(k);
       lo = o < lo ? o : lo;
       hi = o > hi ? o : hi;
+      atomicAdd(&parts[gb_partition(h)], 1u);
     }
   };
   // Head: rows before the first 16-byte aligned key.
@@ -88,6 +94,8 @@ __global__ void __launch_bounds__(256) key_stats_kernel(const int64_t* __restric
   __syncthreads();
   for (int i = threadIdx.x; i < kHllRegs; i += blockDim.x)
     if (r[i]) atomicMax(&out->regs[i], r[i]);
+  for (int i = threadIdx.x; i < (int)kGbParts; i += blockDim.x)
+    if (parts[i]) atomicAdd(&out->parts[i], parts[i]);
 }
 
 static uint64_t hll_estimate(const unsigned int* h, uint64_t n) {
@@ -126,6 +134,7 @@ KeyStats key_stats_i64(Ctx& c, const fdb_dev_column& key, uint64_t n) {
     s.kmin = (int64_t)(h.range[0] ^ (1ull << 63));
     s.kmax = (int64_t)(h.range[1] ^ (1ull << 63));
   }
+  if (n < (1ull << 32)) s.parts.assign(h.parts, h.parts + kGbParts);
   return s;
 }
 

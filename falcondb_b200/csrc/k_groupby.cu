@@ -20,6 +20,7 @@
 //    are atomicMax from a zero identity.  SUM is FP64 atomicAdd (order varies run
 //    to run; tests hold it to 1e-12 relative).
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <type_traits>
 
@@ -1134,6 +1135,334 @@ __global__ void __launch_bounds__(kDenseCompactThreads)
 }
 
 // ===========================================================================
+// 4. int64-key GROUP BY by hash partitions
+// ===========================================================================
+// Many groups, no key much more frequent than another (user ids, hashes): the
+// CTA tables of GbHashOp hold next to none of the keys, and every row costs a
+// probe and four scattered atomics into a global table (20M rows of 1M keys:
+// 0.80 ms, then 0.10 ms to compact 168 MB of table).  Here the rows are first
+// scattered into kGbParts hash partitions, sized exactly by the pass over the
+// keys that also estimates the groups, and one CTA then aggregates a partition in
+// a shared-memory table that holds all its groups and writes them out: 8 + 16 +
+// 16 + 16 bytes per row, and nothing to clear or compact.  20M rows of 1M keys:
+// split 0.145 ms, aggregation 0.32 (at 81 shared-memory wavefronts per 32 rows and
+// 11 of 32 lanes active: the probes, the SUM's compare-and-swap and MIN / MAX of
+// groups of 20 rows diverge).
+struct alignas(16) GbRec {
+  uint64_t key;  // as stored (XOR 2^63)
+  uint64_t val;  // the value's double bits; kNullVal for NULL
+};
+// A NULL value travels as this NaN; a value that has its bits as another one
+// (only that it is NaN shows in any result).
+constexpr uint64_t kNullVal = 0x7FF4DEADBEEF0001ull;
+constexpr int kPartThreads = 512, kPartItems = 8;
+constexpr uint32_t kPartTile = kPartThreads * kPartItems;
+static_assert(kGbParts == kPartThreads, "one thread per partition in a tile's scan");
+
+struct PartCounts {
+  uint32_t n[kGbParts];
+};
+
+// Where the partitions start (off[0 .. kGbParts]), and the same as cursors.
+__global__ void __launch_bounds__(kGbParts) gb_part_offsets_kernel(PartCounts counts, uint32_t* off, uint32_t* cursor) {
+  __shared__ uint32_t sm[32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = counts.n[threadIdx.x];
+  uint32_t x = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  if (lane == 31) sm[warp] = x;
+  __syncthreads();
+  for (uint32_t w = 0; w < warp; ++w) x += sm[w];
+  off[threadIdx.x] = cursor[threadIdx.x] = x - c;
+  if (threadIdx.x == kGbParts - 1) off[kGbParts] = x;
+}
+
+struct GbPartSmem {
+  GbRec rec[kPartTile];
+  uint16_t part[kPartTile];
+  uint32_t count[kGbParts], start[kGbParts], base[kGbParts];
+  uint32_t scan[32];
+  GSlot null[kPartThreads / 32];
+};
+
+// Tiles of 4096 rows: partition by the key's hash, reorder in shared memory,
+// write runs of about 8 records.  Rows with a NULL key are folded per CTA into
+// null_slot.  Bound by shared memory: one atomic and two stores at random places
+// per row.
+__global__ void __launch_bounds__(kPartThreads, 2)
+    gb_part_split_kernel(DevCol key, DevCol val, uint32_t n, uint32_t* cursor, GbRec* __restrict__ out,
+                         GSlot* null_slot, int* err) {
+  extern __shared__ __align__(128) unsigned char part_smem[];
+  GbPartSmem& S = *reinterpret_cast<GbPartSmem*>(part_smem);
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t t0 = blockIdx.x * kPartTile, rows = min(kPartTile, n - t0);
+  const int64_t* keys = static_cast<const int64_t*>(key.values) + t0;
+  const uint64_t* vals = static_cast<const uint64_t*>(val.values) + t0;
+  const bool f64 = val.dtype == FDB_FLOAT64;
+  uint64_t k[kPartItems], v[kPartItems];
+#pragma unroll
+  for (int j = 0; j < kPartItems; ++j) {
+    const uint32_t i = j * kPartThreads + tid;
+    k[j] = v[j] = 0;
+    if (i < rows) {
+      k[j] = (uint64_t)__ldcs(keys + i);
+      v[j] = __ldcs(vals + i);
+    }
+  }
+  S.count[tid] = 0;
+  __syncthreads();
+  GSlot null{0, 0, 0.0, 0, 0};
+  uint32_t pr[kPartItems];  // partition << 16 | arrival number; ~0: not in a partition
+#pragma unroll
+  for (int j = 0; j < kPartItems; ++j) {
+    const uint32_t i = j * kPartThreads + tid;
+    pr[j] = 0xFFFFFFFFu;
+    if (i >= rows) continue;
+    const bool has_v = col_valid(val, t0 + i);
+    const double x = f64 ? __longlong_as_double((long long)v[j]) : (double)(int64_t)v[j];
+    if (!col_valid(key, t0 + i) || (int64_t)k[j] == INT64_MIN) {
+      ++null.count;
+      if (has_v) {
+        null.sum += x;
+        if (!isnan(x)) {
+          const unsigned long long o = f64_ord_key(x);
+          null.nmin = ~o > null.nmin ? ~o : null.nmin;
+          null.max = o > null.max ? o : null.max;
+        }
+      }
+      continue;
+    }
+    k[j] ^= 1ull << 63;
+    v[j] = (uint64_t)__double_as_longlong(x);
+    if (v[j] == kNullVal) v[j] = 0x7FF8000000000000ull;
+    if (!has_v) v[j] = kNullVal;
+    const uint32_t p = gb_partition(mix64(k[j]));
+    pr[j] = p << 16 | atomicAdd(&S.count[p], 1u);
+  }
+  const int any_null = __syncthreads_or(null.count != 0);
+  const uint32_t c = S.count[tid];
+  uint32_t g = 0;
+  if (c) g = atomicAdd(&cursor[tid], c);  // its round trip runs under the scan
+  uint32_t x = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  if (lane == 31) S.scan[warp] = x;
+  __syncthreads();
+  uint32_t s = lane < kPartThreads / 32 ? S.scan[lane] : 0u;
+#pragma unroll
+  for (int o = 1; o < kPartThreads / 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= (uint32_t)o) s += y;
+  }
+  const uint32_t before = __shfl_sync(0xffffffffu, s, warp ? warp - 1 : 0);
+  const uint32_t placed = __shfl_sync(0xffffffffu, s, kPartThreads / 32 - 1);
+  x += (warp ? before : 0u) - c;
+  S.start[tid] = x;
+  S.base[tid] = g - x;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kPartItems; ++j)
+    if (pr[j] != 0xFFFFFFFFu) {
+      const uint32_t p = pr[j] >> 16, at = S.start[p] + (pr[j] & 0xFFFFu);
+      S.rec[at] = GbRec{k[j], v[j]};
+      S.part[at] = (uint16_t)p;
+    }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kPartItems; ++j) {
+    const uint32_t i = j * kPartThreads + tid;
+    if (i < placed) {
+      const uint32_t at = S.base[S.part[i]] + i;
+      if (at < n)
+        out[at] = S.rec[i];
+      else
+        atomicExch(err, kErrCapacity);
+    }
+  }
+  if (any_null) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      null.count += __shfl_xor_sync(0xffffffffu, null.count, o);
+      null.sum += __shfl_xor_sync(0xffffffffu, null.sum, o);
+      null.nmin = max(null.nmin, __shfl_xor_sync(0xffffffffu, null.nmin, o));
+      null.max = max(null.max, __shfl_xor_sync(0xffffffffu, null.max, o));
+    }
+    if (lane == 0) S.null[warp] = null;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < kPartThreads / 32; ++w) {
+        null.count += S.null[w].count;
+        null.sum += S.null[w].sum;
+        null.nmin = max(null.nmin, S.null[w].nmin);
+        null.max = max(null.max, S.null[w].max);
+      }
+      gslot_merge(null_slot, null);
+    }
+  }
+}
+
+// A partition's table, 40 bytes per slot: 4096 slots, one CTA per SM.
+constexpr uint32_t kPartSlots = 4096;
+constexpr int kAggThreads = 1024, kAggRows = 4;
+constexpr uint32_t kPartProbe = 128;
+struct GbPartTab {
+  uint64_t key[kPartSlots];  // 0 = empty
+  double sum[kPartSlots];
+  unsigned long long nmin[kPartSlots], max[kPartSlots];
+  uint32_t mm16[kPartSlots];   // as HTab's
+  uint32_t count[kPartSlots];
+  uint32_t scan[32];
+  uint32_t stack[64][2];       // sub-ranges of the partition still to do: bits, value
+  uint32_t depth, overflow;
+  unsigned long long out0;
+};
+
+// One CTA per partition.  A partition with more groups than its table takes is
+// done in sub-ranges of its hash: one that overflows is split in two by another
+// bit.  sub_bits: the split that the estimated groups suggest to begin with.
+__global__ void __launch_bounds__(kAggThreads) gb_part_agg_kernel(const GbRec* __restrict__ rec, const uint32_t* off,
+                                                                  int sub_bits, const GSlot* null_slot,
+                                                                  fdb_group_i64* out, uint64_t cap_out,
+                                                                  unsigned long long* ngroups, int* err) {
+  extern __shared__ __align__(128) unsigned char part_smem[];
+  GbPartTab& T = *reinterpret_cast<GbPartTab*>(part_smem);
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t r0 = off[blockIdx.x], r1 = off[blockIdx.x + 1];
+  if (tid == 0) {
+    T.depth = 0;
+    for (uint32_t v = 0; v < 1u << sub_bits; ++v) {
+      T.stack[T.depth][0] = sub_bits;
+      T.stack[T.depth++][1] = v;
+    }
+    if (blockIdx.x == 0 && null_slot->count) {
+      const unsigned long long pos = atomicAdd(ngroups, 1ull);
+      if (pos < cap_out)
+        out[pos] = gslot_group(0, *null_slot);  // key INT64_MIN
+      else
+        atomicExch(err, kErrCapacity);
+    }
+  }
+  if (r0 == r1) return;
+  __syncthreads();
+  while (T.depth > 0) {
+    const uint32_t bits = T.stack[T.depth - 1][0], value = T.stack[T.depth - 1][1];
+    const uint64_t low = (1ull << bits) - 1;
+    __syncthreads();
+    if (tid == 0) {
+      --T.depth;
+      T.overflow = 0;
+    }
+    uint4* clear = reinterpret_cast<uint4*>(&T);
+    for (uint32_t i = tid; i < offsetof(GbPartTab, scan) / 16; i += kAggThreads) clear[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    for (uint32_t b = r0; b < r1; b += kAggThreads * kAggRows) {
+      GbRec x[kAggRows];
+#pragma unroll
+      for (int j = 0; j < kAggRows; ++j) {
+        const uint32_t i = b + j * kAggThreads + tid;
+        x[j].key = 0;
+        if (i < r1) x[j] = rec[i];
+      }
+#pragma unroll
+      for (int j = 0; j < kAggRows; ++j) {
+        if (x[j].key == 0) continue;  // past the end: no stored key is zero
+        const uint64_t h = mix64(x[j].key);
+        if ((h & low) != value) continue;
+        uint32_t s = (uint32_t)(h >> 43) & (kPartSlots - 1);  // the bits below the partition's
+        uint32_t probe = 0;
+        for (; probe < kPartProbe; ++probe) {
+          const uint64_t cur = *reinterpret_cast<volatile uint64_t*>(&T.key[s]);
+          if (cur == x[j].key) break;
+          if (cur == 0) {
+            const uint64_t prev = atomicCAS(reinterpret_cast<unsigned long long*>(&T.key[s]), 0ull, x[j].key);
+            if (prev == 0 || prev == x[j].key) break;
+          }
+          s = (s + 1) & (kPartSlots - 1);
+        }
+        if (probe == kPartProbe) {
+          T.overflow = 1;
+          continue;
+        }
+        atomicAdd(&T.count[s], 1u);
+        if (x[j].val == kNullVal) continue;
+        const double v = __longlong_as_double((long long)x[j].val);
+        atomicAdd(&T.sum[s], v);
+        if (isnan(v)) continue;
+        const unsigned long long o = f64_ord_key(v);
+        const uint32_t w = *reinterpret_cast<volatile uint32_t*>(&T.mm16[s]);
+        volatile uint16_t* bound = reinterpret_cast<volatile uint16_t*>(&T.mm16[s]);
+        const uint32_t n16 = (uint32_t)(~o >> 48), o16 = (uint32_t)(o >> 48);
+        if (n16 >= (w & 0xFFFFu) && ~o > *reinterpret_cast<volatile unsigned long long*>(&T.nmin[s])) {
+          atomicMax(&T.nmin[s], ~o);
+          bound[0] = (uint16_t)n16;
+        }
+        if (o16 >= (w >> 16) && o > *reinterpret_cast<volatile unsigned long long*>(&T.max[s])) {
+          atomicMax(&T.max[s], o);
+          bound[1] = (uint16_t)o16;
+        }
+      }
+    }
+    __syncthreads();
+    if (T.overflow) {
+      if (tid == 0) {
+        if (T.depth + 2 > 64 || bits >= 32) {
+          atomicExch(err, kErrCapacity);
+        } else {
+          for (uint32_t v = 0; v < 2; ++v) {
+            T.stack[T.depth][0] = bits + 1;
+            T.stack[T.depth++][1] = value | v << bits;
+          }
+        }
+      }
+      __syncthreads();
+      continue;
+    }
+    // Live slots to the output, in any order.
+    constexpr uint32_t kPer = kPartSlots / kAggThreads;
+    uint32_t live = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < kPer; ++q) live += T.key[q * kAggThreads + tid] != 0;
+    uint32_t x = live;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31) T.scan[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t s = T.scan[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= (uint32_t)o) s += y;
+      }
+      T.scan[lane] = s;
+      if (lane == 31) T.out0 = atomicAdd(ngroups, (unsigned long long)s);
+    }
+    __syncthreads();
+    uint64_t pos = T.out0 + (warp ? T.scan[warp - 1] : 0u) + x - live;
+#pragma unroll
+    for (uint32_t q = 0; q < kPer; ++q) {
+      const uint32_t s = q * kAggThreads + tid;
+      if (T.key[s] == 0) continue;
+      if (pos < cap_out)
+        out[pos] = gslot_group(T.key[s], GSlot{T.key[s], T.count[s], T.sum[s], T.nmin[s], T.max[s]});
+      else
+        atomicExch(err, kErrCapacity);
+      ++pos;
+    }
+    __syncthreads();
+  }
+}
+
+// ===========================================================================
 // Launchers
 // ===========================================================================
 constexpr uint64_t kGbTilesPerCta = 8;
@@ -1370,6 +1699,7 @@ GbSizing group_by_i64_sizing(Ctx& c, const fdb_dev_column& key, uint64_t n, uint
   s.has_range = k.has_range;
   s.kmin = k.kmin;
   s.kmax = k.kmax;
+  s.parts = k.parts;
   return s;
 }
 
@@ -1387,13 +1717,43 @@ static uint64_t gb_dense_slots(const GbSizing& s, double load_factor) {
 
 static double gb_load_factor(double lf) { return (lf <= 0.0 || lf >= 1.0) ? 0.5 : lf; }
 
-size_t group_by_i64_scratch(const GbSizing& s, double load_factor) {
+static size_t group_by_i64_scratch(const GbSizing& s, double load_factor) {
   load_factor = gb_load_factor(load_factor);
   // Each scratch_take rounds up to 256 bytes.
   if (const uint64_t slots = gb_dense_slots(s, load_factor))
     return (slots + 1) * sizeof(DSlot) + (slots / kDenseChunk + 1) * 8 + 3 * 256;
   const uint64_t cap = gb_table_capacity(s.groups ? s.groups : 1, load_factor);
   return (cap + 1) * sizeof(GSlot) + 2 * 256;
+}
+
+// Whether the hash-partition path takes this GROUP BY: no WHERE, a hashed table
+// otherwise, at least 64 groups per partition (with fewer, a CTA's rows meet in
+// few slots: their compare-and-swap sums retry one another), at most two tables'
+// worth of them, and no partition with much more than its share of the rows (a
+// frequent key, whose partition one CTA would have to itself; GbHashOp's CTA
+// tables take such keys in).  Below a million rows the passes' fixed costs win.
+static bool gb_partitions(const GbSizing& s, double load_factor, uint64_t n, int nterms) {
+  if (nterms || n < (1u << 20) || n >= (1ull << 32) || s.parts.size() != kGbParts) return false;
+  if (s.groups < 64ull * kGbParts || s.groups > 2ull * kGbParts * (kPartSlots * 5 / 8)) return false;
+  if (gb_dense_slots(s, gb_load_factor(load_factor))) return false;
+  uint64_t total = 0, most = 0;
+  for (uint32_t c : s.parts) {
+    total += c;
+    most = std::max<uint64_t>(most, c);
+  }
+  return most * kGbParts <= total + total / 2;
+}
+
+static size_t gb_part_scratch(uint64_t n) {
+  return n * sizeof(GbRec) + sizeof(GSlot) + (2 * kGbParts + 1) * 4 + 5 * 256;
+}
+
+void reserve_group_by_i64(Ctx& c, const GbSizing& s, double load_factor, uint64_t n, int nterms) {
+  const size_t tables = group_by_i64_scratch(s, load_factor) + (16u << 20);
+  if (gb_partitions(s, load_factor, n, nterms) &&
+      c.try_scratch(c.scratch_top + std::max(tables, gb_part_scratch(n) + (1u << 20))))
+    return;
+  c.ensure_scratch(tables);
 }
 
 void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& value, uint64_t n,
@@ -1447,6 +1807,32 @@ void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& va
     FDB_CUDA(cudaGetLastError());
     dense_emit_kernel<<<(unsigned)nchunks, kDenseCompactThreads, 0, c.stream>>>(table, slots, sz.kmin, chunk_off,
                                                                                d_groups, capacity, c.d_err);
+    FDB_CUDA(cudaGetLastError());
+    return;
+  }
+
+  if (gb_partitions(sz, load_factor, n, nterms) && c.scratch_top + gb_part_scratch(n) <= c.scratch.bytes) {
+    GbRec* rec = static_cast<GbRec*>(c.scratch_take(n * sizeof(GbRec)));
+    GSlot* null_slot = static_cast<GSlot*>(c.scratch_take(sizeof(GSlot)));
+    uint32_t* off = static_cast<uint32_t*>(c.scratch_take((kGbParts + 1) * 4));
+    uint32_t* cursor = static_cast<uint32_t*>(c.scratch_take(kGbParts * 4));
+    FDB_CUDA(cudaMemsetAsync(null_slot, 0, sizeof(GSlot), c.stream));
+    FDB_CUDA(cudaMemsetAsync(d_ngroups, 0, 8, c.stream));
+    static PerDeviceOnce attr;
+    attr(c.device, [&] {
+      FDB_CUDA(cudaFuncSetAttribute(gb_part_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(GbPartSmem)));
+      FDB_CUDA(cudaFuncSetAttribute(gb_part_agg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)sizeof(GbPartTab)));
+    });
+    PartCounts counts;
+    std::copy(sz.parts.begin(), sz.parts.end(), counts.n);
+    gb_part_offsets_kernel<<<1, kGbParts, 0, c.stream>>>(counts, off, cursor);
+    gb_part_split_kernel<<<(unsigned)((n + kPartTile - 1) / kPartTile), kPartThreads, sizeof(GbPartSmem), c.stream>>>(
+        dcols[0], dcols[1], (uint32_t)n, cursor, rec, null_slot, c.d_err);
+    const int sub_bits = sz.groups > (uint64_t)kGbParts * (kPartSlots * 5 / 8) ? 1 : 0;
+    gb_part_agg_kernel<<<kGbParts, kAggThreads, sizeof(GbPartTab), c.stream>>>(
+        rec, off, sub_bits, null_slot, d_groups, capacity, reinterpret_cast<unsigned long long*>(d_ngroups), c.d_err);
     FDB_CUDA(cudaGetLastError());
     return;
   }

@@ -1068,7 +1068,7 @@ static void run_aggregates(Plan& plan, const Rel& rel, const Query& q, fdb_resul
       plan.c.scratch_reset();
       const GbSizing sz = group_by_i64_sizing(plan.c, col.dev, rel.nrows, 0);
       plan.c.scratch_reset();
-      plan.c.ensure_scratch(group_by_i64_scratch(sz, 0.5) + (16u << 20));
+      reserve_group_by_i64(plan.c, sz, 0.5, rel.nrows, (int)prog.size());
       op_group_by_i64(plan.c, col.dev, col.dev, rel.nrows, prog.data(), (int)prog.size(), pcols.data(),
                       (int)pcols.size(), sz, 0.5, d, cap, dn);
       plan.check();
@@ -1215,7 +1215,7 @@ static void run_group_by(Plan& plan, const Rel& rel, const Query& q, fdb_result*
     std::vector<fdb_group_i64> groups;
     if (rel.nrows > 0) {
       const GbSizing sz = group_by_i64_sizing(plan.c, key.dev, rel.nrows, 0);
-      plan.c.ensure_scratch(group_by_i64_scratch(sz, 0.5) + (16u << 20));
+      reserve_group_by_i64(plan.c, sz, 0.5, rel.nrows, (int)prog.size());
       op_group_by_i64(plan.c, key.dev, rel.cols[vc].dev, rel.nrows, prog.data(), (int)prog.size(), pcols.data(),
                       (int)pcols.size(), sz, 0.5, d, cap, dn);
       plan.check();
