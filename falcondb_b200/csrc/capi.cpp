@@ -58,6 +58,7 @@ Ctx::~Ctx() {
   tables.clear();
   if (scratch.ptr) cudaFree(scratch.ptr);
   if (d_err) cudaFree(d_err);
+  if (landing) cudaFreeHost(landing);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (stream) cudaStreamDestroy(stream);
@@ -135,10 +136,31 @@ void* Ctx::scratch_take(size_t bytes) {
   return p;
 }
 
-int Ctx::check_device_error() {
-  FDB_CUDA(cudaStreamSynchronize(stream));
+void HostReads::add(void* host, const void* dev, size_t bytes) {
+  if (bytes == 0) return;
+  if (n_ < kItems && bytes <= Ctx::kLandingBytes - top_) {
+    FDB_CUDA(cudaMemcpyAsync(c_.landing + top_, dev, bytes, cudaMemcpyDeviceToHost, c_.stream));
+    items_[n_++] = Item{host, top_, bytes};
+    top_ += (bytes + 15) & ~size_t(15);
+    if (top_ > Ctx::kLandingBytes) top_ = Ctx::kLandingBytes;
+  } else {
+    FDB_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c_.stream));
+  }
+}
+
+void HostReads::wait() {
+  FDB_CUDA(cudaStreamSynchronize(c_.stream));
+  for (int i = 0; i < n_; ++i) std::memcpy(items_[i].host, c_.landing + items_[i].off, items_[i].bytes);
+  n_ = 0;
+  top_ = 0;
+}
+
+int Ctx::check_device_error(HostReads* also) {
+  HostReads own(*this);
+  HostReads& r = also ? *also : own;
   int e = 0;
-  FDB_CUDA(cudaMemcpy(&e, d_err, sizeof(int), cudaMemcpyDeviceToHost));
+  r.add(&e, d_err, sizeof(int));
+  r.wait();
   if (e) {
     // Clear the error word and the ticket so the context stays usable.
     FDB_CUDA(cudaMemset(d_err, 0, kTicketBytes));
@@ -235,6 +257,9 @@ int fdb_open(int device, uint64_t mem_budget_bytes, fdb_db** out) {
     FDB_CUDA(cudaStreamSynchronize(c.stream));
     c.d_ticket = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(c.d_err) + 64);
     c.ensure_scratch(default_scratch(c));
+    void* landing = nullptr;
+    FDB_CUDA(cudaMallocHost(&landing, Ctx::kLandingBytes));
+    c.landing = static_cast<char*>(landing);
   });
   if (rc == FDB_OK) *out = db.release();
   return rc;

@@ -74,6 +74,8 @@ struct LaunchCfg {
   int threads = 0;     // threads per CTA
 };
 
+class HostReads;
+
 struct Ctx {
   int device = 0;
   int sm_count = 0;
@@ -92,6 +94,9 @@ struct Ctx {
   static constexpr size_t kTicketBytes = 256;
   DevBuf scratch;
   size_t scratch_top = kTicketBytes;
+  // Page-locked landing area of the words that an operator reads back (HostReads).
+  static constexpr size_t kLandingBytes = 64 * 1024;
+  char* landing = nullptr;
   int* d_err = nullptr;                  // deferred device error word (in scratch head)
   unsigned int* d_ticket = nullptr;      // last-CTA ticket (in scratch head)
 
@@ -114,7 +119,33 @@ struct Ctx {
   // and nothing changes, when it would take more than a quarter of what the
   // budget has left or the device has no room for it.
   bool try_scratch(size_t bytes);
-  int check_device_error();                      // reads and clears d_err (syncs)
+  // Reads and clears d_err (syncs), with what `also` has queued in the same wait.
+  int check_device_error(HostReads* also = nullptr);
+};
+
+// Copies of device results to the host, queued on the operator stream and
+// delivered by one wait.  A copy into pageable memory is staged by the driver
+// and waited for by itself (16 to 33 us each on the host); those that fit land in
+// the context's page-locked buffer instead.  One object at a time per context,
+// under the context's lock; `host` must live until wait().
+class HostReads {
+ public:
+  explicit HostReads(Ctx& ctx) : c_(ctx) {}
+  HostReads(const HostReads&) = delete;
+  HostReads& operator=(const HostReads&) = delete;
+  void add(void* host, const void* dev, size_t bytes);
+  void wait();
+
+ private:
+  struct Item {
+    void* host;
+    size_t off, bytes;
+  };
+  static constexpr int kItems = 8;
+  Ctx& c_;
+  Item items_[kItems];
+  int n_ = 0;
+  size_t top_ = 0;
 };
 
 // Converts the C view to the kernel view.

@@ -126,8 +126,9 @@ KeyStats key_stats_i64(Ctx& c, const fdb_dev_column& key, uint64_t n) {
                                                key.validity_offset, n, d);
   FDB_CUDA(cudaGetLastError());
   KeyStatsOut h;
-  FDB_CUDA(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
-  FDB_CUDA(cudaStreamSynchronize(c.stream));
+  HostReads reads(c);
+  reads.add(&h, d, sizeof(h));
+  reads.wait();
   s.distinct = n <= 4096 ? n : hll_estimate(h.regs, n);
   if (h.range[0] <= h.range[1]) {
     s.has_range = true;

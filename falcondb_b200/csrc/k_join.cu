@@ -387,8 +387,9 @@ HashTable* op_join_build(Ctx& c, const fdb_dev_column& key, const fdb_dev_column
                                                          key.validity_offset, n, range);
     FDB_CUDA(cudaGetLastError());
     unsigned long long hr[2] = {0, 0};
-    FDB_CUDA(cudaMemcpyAsync(hr, range, 16, cudaMemcpyDeviceToHost, c.stream));
-    FDB_CUDA(cudaStreamSynchronize(c.stream));
+    HostReads reads(c);
+    reads.add(hr, range, 16);
+    reads.wait();
     if (hr[1] != 0) {
       const uint64_t kmin = ~hr[0] ^ (1ull << 63), kmax = hr[1] ^ (1ull << 63);  // two's complement bits
       // Both kinds keep the range: a hashed table uses it as a min/max filter
@@ -437,8 +438,9 @@ HashTable* op_join_build(Ctx& c, const fdb_dev_column& key, const fdb_dev_column
   }
   FDB_CUDA(cudaGetLastError());
   unsigned int hdup = 0;
-  FDB_CUDA(cudaMemcpyAsync(&hdup, dup, 4, cudaMemcpyDeviceToHost, c.stream));
-  const int e = c.check_device_error();  // synchronises the stream
+  HostReads reads(c);
+  reads.add(&hdup, dup, 4);
+  const int e = c.check_device_error(&reads);  // synchronises the stream
   if (e) {
     join_free(h.release());
     fail(e, "join build failed on the device");

@@ -573,8 +573,9 @@ static NullSplit split_nulls(Ctx& c, const DevCol& dc, uint64_t n) {
   sort_valid_mask_kernel<<<g, 256, 0, c.stream>>>(dc, n, true, mask);
   op_compact_mask(c, mask, n, r.nulls, n, r.d_counts + 1);
   uint64_t hc[2] = {0, 0};
-  FDB_CUDA(cudaMemcpyAsync(hc, r.d_counts, 16, cudaMemcpyDeviceToHost, c.stream));
-  FDB_CUDA(cudaStreamSynchronize(c.stream));
+  HostReads reads(c);
+  reads.add(hc, r.d_counts, 16);
+  reads.wait();
   if (hc[0] + hc[1] != n) fail(FDB_E_GENERIC, "sort: valid and NULL rows do not add up to the row count");
   r.m = hc[0];
   r.nnull = hc[1];
@@ -618,8 +619,9 @@ static void radix_sort_pairs(Ctx& c, uint32_t m, KeysFn keys_fn, uint32_t* rows_
     FDB_CUDA(cudaMemsetAsync(run.vary, 0, 16, c.stream));
     keys_fn(run.ka, run.va, run.vary, nullptr);
     FDB_CUDA(cudaGetLastError());
-    FDB_CUDA(cudaMemcpyAsync(run.hv, run.vary, 16, cudaMemcpyDeviceToHost, c.stream));
-    FDB_CUDA(cudaStreamSynchronize(c.stream));
+    HostReads reads(c);
+    reads.add(run.hv, run.vary, 16);
+    reads.wait();
   }
   uint64_t *ka = run.ka, *kb = run.kb;
   uint32_t *va = run.va, *vb = run.vb, *hist = run.hist, *bsum = run.bsum;
@@ -788,8 +790,9 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
   uint32_t host[36] = {};
   auto read_states = [&] {
     FDB_CUDA(cudaGetLastError());
-    FDB_CUDA(cudaMemcpyAsync(host, state, sizeof(host), cudaMemcpyDeviceToHost, c.stream));
-    FDB_CUDA(cudaStreamSynchronize(c.stream));
+    HostReads reads(c);
+    reads.add(host, state, sizeof(host));
+    reads.wait();
   };
   read_states();
   if (host[kMsdRepeats]) {
@@ -1194,8 +1197,9 @@ void op_sort_multi(Ctx& c, const SortKey* keys, int nkeys, const uint32_t* d_lis
       mkey_null_mask_kernel<<<gw, 256, 0, c.stream>>>(mk, d_list, d_pos, n, true, reinterpret_cast<uint32_t*>(mask));
       op_compact_mask(c, mask, n, nidx, n, cnt + 1);
       uint64_t hc[2] = {0, 0};
-      FDB_CUDA(cudaMemcpyAsync(hc, cnt, 16, cudaMemcpyDeviceToHost, c.stream));
-      FDB_CUDA(cudaStreamSynchronize(c.stream));
+      HostReads reads(c);
+      reads.add(hc, cnt, 16);
+      reads.wait();
       if (hc[0] + hc[1] != n) fail(FDB_E_GENERIC, "sort: valid and NULL positions do not add up");
       mv = hc[0];
       mnull = hc[1];

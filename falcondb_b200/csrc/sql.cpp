@@ -572,17 +572,31 @@ struct Plan {
   template <typename T>
   std::vector<T> to_host(const T* d, size_t n) {
     std::vector<T> h(n);
-    if (n) FDB_CUDA(cudaMemcpyAsync(h.data(), d, n * sizeof(T), cudaMemcpyDeviceToHost, c.stream));
-    FDB_CUDA(cudaStreamSynchronize(c.stream));
+    HostReads reads(c);
+    reads.add(h.data(), d, n * sizeof(T));
+    reads.wait();
     return h;
   }
   template <typename T>
   T one(const T* d) {
     return to_host(d, 1)[0];
   }
-  void check() {
-    const int e = c.check_device_error();
+  void check(HostReads* also = nullptr) {
+    const int e = c.check_device_error(also);
     if (e) fail(e, e == FDB_E_TIMEOUT ? "a device-side wait timed out" : "an operator output overflowed");
+  }
+  // check(), and results in the same wait.
+  template <typename T>
+  std::vector<T> checked(const T* d, size_t n) {
+    std::vector<T> h(n);
+    HostReads reads(c);
+    reads.add(h.data(), d, n * sizeof(T));
+    check(&reads);
+    return h;
+  }
+  template <typename T>
+  T checked_one(const T* d) {
+    return checked(d, 1)[0];
   }
 };
 
@@ -811,9 +825,12 @@ static void fetch_rows(Plan& plan, const Rel& r, int rc, const uint32_t* d_rows,
   uint64_t* d_valid = nullptr;
   if (col.dev.validity) d_valid = plan.dev<uint64_t>((n + 63) / 64);
   op_gather(plan.c, col.dev, d_rows, n, d_vals, d_valid);
-  std::vector<uint8_t> raw = plan.to_host(static_cast<uint8_t*>(d_vals), n * esz);
-  std::vector<uint64_t> vw;
-  if (d_valid) vw = plan.to_host(d_valid, (n + 63) / 64);
+  std::vector<uint8_t> raw(n * esz);
+  std::vector<uint64_t> vw(d_valid ? (n + 63) / 64 : 0);
+  HostReads reads(plan.c);
+  reads.add(raw.data(), d_vals, raw.size());
+  reads.add(vw.data(), d_valid, vw.size() * 8);
+  reads.wait();
   out.nulls.assign(n, 0);
   if (col.dtype == FDB_INT64 || col.dtype == FDB_FLOAT64) {
     if (col.dtype == FDB_INT64) {
@@ -956,8 +973,7 @@ static void run_aggregates(Plan& plan, const Rel& rel, const Query& q, fdb_resul
       res->cols[0].i64.push_back((int64_t)rel.nrows);
     } else {
       op_filter_count(plan.c, cols.data(), (int)cols.size(), rel.nrows, prog.data(), (int)prog.size(), d);
-      plan.check();
-      res->cols[0].i64.push_back((int64_t)plan.one(d));
+      res->cols[0].i64.push_back((int64_t)plan.checked_one(d));
     }
     res->cols[0].nulls.push_back(0);
     res->rows = 1;
@@ -1020,8 +1036,7 @@ static void run_aggregates(Plan& plan, const Rel& rel, const Query& q, fdb_resul
     }
     op_aggregate(plan.c, cols.data(), (int)cols.size(), rel.nrows, prog.data(), (int)prog.size(), specs.data(),
                  (int)specs.size(), d);
-    plan.check();
-    std::vector<fdb_agg_value> h = plan.to_host(d, specs.size());
+    std::vector<fdb_agg_value> h = plan.checked(d, specs.size());
     for (size_t k = 0; k < specs.size(); ++k) {
       auto& col = res->cols[which[k]];
       if (col.dtype == FDB_INT64) {
@@ -1053,8 +1068,7 @@ static void run_aggregates(Plan& plan, const Rel& rel, const Query& q, fdb_resul
       const uint32_t dl = (uint32_t)col.dict->size();
       uint64_t* d = plan.dev<uint64_t>((dl + 63) / 64);
       op_distinct_codes(plan.c, cols.data(), (int)cols.size(), rel.nrows, prog.data(), (int)prog.size(), lc, dl, d);
-      plan.check();
-      std::vector<uint64_t> bits = plan.to_host(d, (dl + 63) / 64);
+      std::vector<uint64_t> bits = plan.checked(d, (dl + 63) / 64);
       std::set<std::string> seen;  // DistinctSet::Strings over the present codes
       for (uint32_t code = 0; code < dl; ++code)
         if ((bits[code >> 6] >> (code & 63)) & 1ull) seen.insert((*col.dict)[code]);
@@ -1071,8 +1085,7 @@ static void run_aggregates(Plan& plan, const Rel& rel, const Query& q, fdb_resul
       reserve_group_by_i64(plan.c, sz, 0.5, rel.nrows, (int)prog.size());
       op_group_by_i64(plan.c, col.dev, col.dev, rel.nrows, prog.data(), (int)prog.size(), pcols.data(),
                       (int)pcols.size(), sz, 0.5, d, cap, dn);
-      plan.check();
-      const uint64_t ng = plan.one(dn);
+      const uint64_t ng = plan.checked_one(dn);
       std::vector<fdb_group_i64> g = plan.to_host(d, ng);
       for (auto& x : g)
         if (!(x.key == INT64_MIN)) ++result;  // NULL is not a distinct value
@@ -1160,12 +1173,12 @@ static void run_group_by(Plan& plan, const Rel& rel, const Query& q, fdb_result*
       if (rel.nrows > 0) {
         op_group_by_codes(plan.c, cols.data(), (int)cols.size(), rel.nrows, prog.data(), (int)prog.size(), klc, dl,
                           specs.data(), (int)specs.size(), d, dr);
-        plan.check();
-        std::vector<fdb_agg_value> h = plan.to_host(d, (size_t)ng * specs.size());
-        if (!rows_known) {
-          group_rows = plan.to_host(dr, ng);
-          rows_known = true;
-        }
+        std::vector<fdb_agg_value> h((size_t)ng * specs.size());
+        HostReads reads(plan.c);
+        reads.add(h.data(), d, h.size() * sizeof(fdb_agg_value));
+        if (!rows_known) reads.add(group_rows.data(), dr, ng * sizeof(int64_t));
+        rows_known = true;
+        plan.check(&reads);
         for (size_t k = 0; k < which.size(); ++k) {
           vals[which[k]].resize(ng);
           for (uint32_t g = 0; g < ng; ++g) vals[which[k]][g] = h[(size_t)g * specs.size() + k];
@@ -1218,8 +1231,7 @@ static void run_group_by(Plan& plan, const Rel& rel, const Query& q, fdb_result*
       reserve_group_by_i64(plan.c, sz, 0.5, rel.nrows, (int)prog.size());
       op_group_by_i64(plan.c, key.dev, rel.cols[vc].dev, rel.nrows, prog.data(), (int)prog.size(), pcols.data(),
                       (int)pcols.size(), sz, 0.5, d, cap, dn);
-      plan.check();
-      groups = plan.to_host(d, plan.one(dn));
+      groups = plan.to_host(d, plan.checked_one(dn));
     }
     for (const fdb_group_i64& g : groups) {
       if (g.count <= 0) continue;
@@ -1291,8 +1303,7 @@ static void emit_rows(Plan& plan, const Rel& rel, const std::vector<int>& outcol
     plan.c.scratch_reset();
     op_distinct_multi(plan.c, cols.data(), ranks.data(), rank_lens.data(), (int)cols.size(), d_list, n, pos, dcount);
     plan.c.scratch_reset();
-    plan.check();
-    const uint64_t k = plan.one(dcount);
+    const uint64_t k = plan.checked_one(dcount);
     uint32_t* kept = pos;
     if (d_list) {
       kept = plan.dev<uint32_t>(std::max<uint64_t>(k, 1));
@@ -1321,8 +1332,7 @@ static void emit_rows(Plan& plan, const Rel& rel, const std::vector<int>& outcol
     uint64_t* dcount = plan.dev<uint64_t>(1);
     op_distinct(plan.c, g, n, pos, dcount);
     plan.c.scratch_reset();  // the sort's working memory is free for the next operator
-    plan.check();
-    const uint64_t k = plan.one(dcount);
+    const uint64_t k = plan.checked_one(dcount);
     uint32_t* kept = pos;
     if (d_list) {
       kept = plan.dev<uint32_t>(std::max<uint64_t>(k, 1));
@@ -1411,8 +1421,7 @@ static void run_projection(Plan& plan, const Rel& rel_in, const Query& q, fdb_re
     d_rows = plan.dev<uint32_t>(n);
     uint64_t* dc = plan.dev<uint64_t>(1);
     op_compact_mask(plan.c, mask, n, d_rows, n, dc);
-    plan.check();
-    nsel = plan.one(dc);
+    nsel = plan.checked_one(dc);
     all_rows = false;
   }
 
@@ -1475,8 +1484,7 @@ static void run_projection(Plan& plan, const Rel& rel_in, const Query& q, fdb_re
         rows_col.values = d_rows;
         op_gather(plan.c, rows_col, local_top, k, top, nullptr);
       }
-      plan.check();
-      const uint64_t got = plan.one(dcount);
+      const uint64_t got = plan.checked_one(dcount);
       emit_rows(plan, rel, outcols, q, top, got, res);
       return;
     }
@@ -1665,8 +1673,7 @@ static void run_join(Plan& plan, Query& q, const JoinSpec& js, fdb_result* res) 
     const fdb_dev_column* val = (semi_anti && sum_col >= 0) ? &lrel.cols[sum_col].dev : nullptr;
     c.scratch_reset();
     op_join_probe_agg(c, *ht, lkey, val, L.nrows, js.type, d);
-    plan.check();
-    const fdb_join_agg h = plan.one(d);
+    const fdb_join_agg h = plan.checked_one(d);
     for (const SelItem& it : q.items) {
       if (it.agg == FDB_AGG_COUNT_STAR) {
         push_col(res, out_name(it), FDB_INT64);
@@ -1689,15 +1696,13 @@ static void run_join(Plan& plan, Query& q, const JoinSpec& js, fdb_result* res) 
   fdb_join_agg* dcnt = plan.dev<fdb_join_agg>(1);
   op_join_probe_agg(c, *ht, lkey, nullptr, L.nrows,
                     semi_anti ? js.type : (js.type == FDB_JOIN_LEFT ? FDB_JOIN_LEFT : FDB_JOIN_INNER), dcnt);
-  plan.check();
-  const uint64_t npairs = (uint64_t)plan.one(dcnt).count;
+  const uint64_t npairs = (uint64_t)plan.checked_one(dcnt).count;
   uint32_t* dl = plan.dev<uint32_t>(npairs);
   uint32_t* dr = semi_anti ? nullptr : plan.dev<uint32_t>(npairs);
   uint64_t* dn = plan.dev<uint64_t>(1);
   c.scratch_reset();
   op_join_probe_pairs(c, *ht, lkey, L.nrows, js.type, dl, dr, npairs, dn);
-  plan.check();
-  const uint64_t got = plan.one(dn);
+  const uint64_t got = plan.checked_one(dn);
   if (got != npairs) fail(FDB_E_GENERIC, "join pair count changed between passes");
   // Pair order from the device is unspecified: order by (left row, right row)
   // so the joined relation is deterministic (the reference probes left rows in
