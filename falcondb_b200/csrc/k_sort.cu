@@ -706,7 +706,13 @@ static MsdPlan msd_plan(uint64_t m) {
     p.parts2 = pow2((m + kMsdFirst * kMsdLeafRows - 1) / (kMsdFirst * kMsdLeafRows));
     p.cap2 = leaf_cap(m / ((uint64_t)kMsdFirst * p.parts2));
   }
-  p.samples = m >= 1024 * kMsdSampleItems ? 1024 * kMsdSampleItems : 2048;
+  // A leaf's size varies with the shares that both levels' samples give it.  With
+  // 32 samples per first-level bucket some bucket of 256 is 1.7 times the average,
+  // and where a leaf has few samples of its own (64 from 128 parts on) one in 10 to
+  // 100 sorts of 100M keys then overflowed a leaf, at the price of a radix sort
+  // (9.5 ms instead of 2.5).  With twice the samples there (1.4 times) a leaf's
+  // capacity is seven of its standard deviations away.
+  p.samples = p.parts2 >= 64 ? 2048 * kMsdSampleItems : m >= 1024 * kMsdSampleItems ? 1024 * kMsdSampleItems : 2048;
   const uint64_t leaves = (uint64_t)p.parts1 * std::max(1u, p.parts2);
   // Pairs of both levels, the maps, counters and offsets, and 256-byte rounding.
   p.bytes = (size_t)p.parts1 * p.cap1 * 12 + (size_t)p.parts1 * p.parts2 * p.cap2 * 12 + leaves * 44 +
@@ -743,7 +749,8 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
     auto set = [](const void* f, size_t bytes) {
       FDB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     };
-    set((const void*)msd_sample_kernel<Src>, sizeof(MsdSampleSmem));
+    set((const void*)msd_sample_kernel<Src, kMsdSampleItems>, sizeof(MsdSampleSmem));
+    set((const void*)msd_sample_kernel<Src, 2 * kMsdSampleItems>, sizeof(MsdSampleSmem));
     set((const void*)msd_split_kernel<Src, false>, sizeof(MsdSplitSmem));
     set((const void*)msd_split_kernel<Src, true>, sizeof(MsdSplitSmem));
     set((const void*)msd_leaf_kernel<Src, false>, sizeof(MsdLeafSmem<kMsdLeafItems>));
@@ -777,10 +784,14 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
   // Two radix passes beat the sample sort at any size, three up to a few million
   // pairs (1.9M int64 keys of 18 bits: 179 us against 204; 20M: 760 against 600).
   const int few_bytes = m < 4'000'000 ? 3 : 2;
-  const uint32_t run = (uint32_t)std::max<uint64_t>(3, 1024ull * p.samples / m);
+  const uint32_t run = (uint32_t)std::max<uint64_t>(3, 1024ull * std::min<uint32_t>(p.samples, 1024 * kMsdSampleItems) / m);
   auto log2 = [](uint32_t x) { return 31 - __builtin_clz(x); };
-  msd_sample_kernel<Src><<<1, 1024, sizeof(MsdSampleSmem), c.stream>>>(src, m, log2(p.samples), p.parts1, run, few_bytes,
-                                                                      map1, state);
+  if (p.samples > 1024 * kMsdSampleItems)
+    msd_sample_kernel<Src, 2 * kMsdSampleItems><<<1, 1024, sizeof(MsdSampleSmem), c.stream>>>(
+        src, m, log2(p.samples), p.parts1, run, few_bytes, map1, state);
+  else
+    msd_sample_kernel<Src, kMsdSampleItems><<<1, 1024, sizeof(MsdSampleSmem), c.stream>>>(
+        src, m, log2(p.samples), p.parts1, run, few_bytes, map1, state);
   // The radix passes' key kernel runs only when the sample showed repeats; one
   // copy then tells the host which way to go.
   const size_t mark = c.scratch_top;

@@ -9,7 +9,7 @@
 // stable, because pairs are compared by (key, position) in the last one, so a
 // pair's place in its tile is the return value of one shared-memory atomic.
 //
-//   msd_sample_kernel   one CTA: up to 8192 sampled keys give the bucket map, a
+//   msd_sample_kernel   one CTA: up to 16384 sampled keys give the bucket map, a
 //                       table over 4096 equal steps of the sample's range (its
 //                       tails cut off) with about the same share of the samples
 //                       in every bucket.  Keys that repeat too often for the
@@ -280,7 +280,7 @@ __device__ __forceinline__ uint32_t msd_build_map(MsdMapSmem& S, const uint64_t 
 constexpr uint32_t kMsdSeen = 2 * 1024 * kMsdSampleItems;  // hash slots of the equal-sample check
 struct MsdSampleSmem {
   MsdMapSmem map;
-  uint64_t keys[1024 * kMsdSampleItems];  // sample tid * kMsdSampleItems + i at i * 1024 + tid
+  uint64_t keys[1024 * kMsdSampleItems];  // thread tid's sample i at i * 1024 + tid
   uint16_t seen[kMsdSeen];
   uint32_t count[kMsdSeen / 8];
   uint32_t equal;
@@ -288,12 +288,16 @@ struct MsdSampleSmem {
 };
 static_assert(kMsdSeen == 1u << 14, "hash bits of the equal-sample check");
 
-template <class Src>
+//
+// kItems samples per thread: the equal-sample check takes the first
+// kMsdSampleItems of them, the map all.
+template <class Src, int kItems>
 __global__ void __launch_bounds__(1024) msd_sample_kernel(Src src, uint32_t m, int log_samples, uint32_t parts,
                                                           uint32_t run, int few_bytes, MsdMap* map, uint32_t* state) {
   extern __shared__ __align__(128) unsigned char msd_smem[];
   MsdSampleSmem& S = *reinterpret_cast<MsdSampleSmem*>(msd_smem);
-  constexpr int kItems = kMsdSampleItems;
+  constexpr int kChecked = kMsdSampleItems;
+  static_assert(kItems >= kChecked, "the check's samples are among the map's");
   const uint32_t tid = threadIdx.x, samples = 1u << log_samples, per = samples / kItems;  // threads with samples
   const bool in = tid < per;
   uint64_t k[kItems];
@@ -343,8 +347,9 @@ __global__ void __launch_bounds__(1024) msd_sample_kernel(Src src, uint32_t m, i
     return;
   }
 #pragma unroll
-  for (int i = 1; i < kItems; ++i) k[i] = in ? src.key(msd_sample_pos(tid * kItems + i, log_samples, m)) : 0;
-  check(std::integral_constant<int, 1>(), std::integral_constant<int, kItems>());
+  for (int i = 1; i < kItems; ++i)
+    k[i] = in ? src.key(msd_sample_pos(tid * kItems + i, log_samples, m)) : 0;
+  check(std::integral_constant<int, 1>(), std::integral_constant<int, kChecked>());
   stop = __syncthreads_or(heavy);
   if (stop || S.equal > limit) {
     if (tid == 0) state[kMsdRepeats] = 1;

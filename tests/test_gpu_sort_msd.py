@@ -110,3 +110,14 @@ def test_sort_within_a_small_budget():
         assert np.array_equal(got, np.argsort(-v, kind="stable"))
         small.synchronize()
         assert small.memory_stats()["in_use"] < 160 << 20
+
+
+@pytest.mark.parametrize("n", [13_107_200, 13_107_201])
+@pytest.mark.parametrize("kind", ["uniform", "spread"])
+def test_sort_around_the_larger_sample(db, n, kind):
+    """From 64 second-level buckets on the first level's map has twice the samples."""
+    v = torch.from_numpy(column(kind, n, np.random.default_rng(n))).cuda()
+    got = ops.sort(db, v, n, False, nulls_last=False).to(torch.int64) & 0xFFFFFFFF
+    bits = v.view(torch.int64)
+    key = torch.where(bits < 0, ~bits ^ torch.iinfo(torch.int64).min, bits)
+    assert bool((got == torch.sort(key, stable=True).indices).all())
