@@ -150,6 +150,44 @@ __device__ __forceinline__ fdb_group_i64 gslot_group(uint64_t skey, const GSlot&
   return g;
 }
 
+// The lanes of a warp whose rows go to the same CTA slot (j; -1: none), merged
+// before the shared-memory atomics: the first of them gets their number and the
+// sum of their values, the others 0 rows.  All 32 lanes call.
+struct SlotRows {
+  uint32_t rows;
+  double sum;
+};
+__device__ __forceinline__ SlotRows warp_slot_rows(int j, double v, int lane) {
+  const unsigned peers = __match_any_sync(0xffffffffu, j >= 0 ? j : -1 - lane);
+  const unsigned below = peers & ((1u << lane) - 1u);
+  unsigned above = peers & ~((2u << lane) - 1u);
+  uint32_t rank = __popc(below);
+  SlotRows r;
+  r.rows = below ? 0u : (uint32_t)__popc(peers);
+  r.sum = v;
+  while (__any_sync(0xffffffffu, above != 0)) {  // halves every group's live lanes
+    const double x = __shfl_sync(0xffffffffu, r.sum, above ? __ffs(above) - 1 : lane);
+    if (above) r.sum += x;
+    above &= __ballot_sync(0xffffffffu, (rank & 1u) == 0);
+    rank >>= 1;
+  }
+  if (j < 0) r.rows = 0;
+  return r;
+}
+
+// Whether a warp's rows are worth merging: at least kMergeLanes of them meet
+// another row in their slot.  Lanes of one slot retry its SUM one after another,
+// while merging costs every row a match and a few shuffles: 30M rows of 64
+// queries with 2000 Zipf(1.1) keys (8 lanes) 790 us without it, 612 with; 50 Zipf
+// keys 995 and 310; one key 3630 and 294; 5M rows of 200 uniform keys (2 lanes) 76
+// without, 89 with.  The line lies between, where neither side is far ahead (3 and
+// 5 differ by 4 us on the last, 0 on the others).
+constexpr int kMergeLanes = 5;
+__device__ __forceinline__ bool warp_slots_repeat(int j, int lane) {
+  const unsigned peers = __match_any_sync(0xffffffffu, j >= 0 ? j : -1 - lane);
+  return __popc(__ballot_sync(0xffffffffu, (peers & ((1u << lane) - 1u)) != 0)) >= kMergeLanes;
+}
+
 // ---------------------------------------------------------------------------
 // CTA table keyed by 64-bit keys, structure of arrays: kSmemSlots slots and the
 // NULL group's (the last).
@@ -159,11 +197,12 @@ __device__ __forceinline__ fdb_group_i64 gslot_group(uint64_t skey, const GSlot&
 //     memory, only when the value improves on the slot.  The first test reads one
 //     word of lower bounds of both order keys' top 16 bits, stored after the keys
 //     are raised (a store that loses a race only lowers a bound).
-// The FLOAT64 SUM stays a compare-and-swap loop, and where keys are skewed it is
-// what costs most: one table of 4096 slots per SM, which takes in every row of
-// 2000 Zipf(1.1) keys, is slower than three of 1024 that send a third of them to
-// the global table (1.5 against 0.84 ms for 30M rows), and columns of sums per
-// thread for the six most frequent keys brought it to 1.0 only.
+// The FLOAT64 SUM stays a compare-and-swap loop; where keys are skewed a warp's
+// rows are merged first (warp_slot_rows).  Without that it was what cost most: one
+// table of 4096 slots per SM, which takes in every row of 2000 Zipf(1.1) keys, was
+// slower than three of 1024 that send a third of them to the global table (1.5
+// against 0.84 ms for 30M rows), and columns of sums per thread for the six most
+// frequent keys brought it to 1.0 only.
 // ---------------------------------------------------------------------------
 struct HTab {
   uint64_t key[kSmemSlots + 1];             // 0 = empty
@@ -196,11 +235,13 @@ __device__ __forceinline__ int htab_slot(HTab& t, uint64_t skey) {
   return -1;
 }
 
-__device__ __forceinline__ void htab_accum(HTab& t, uint32_t j, double v, bool has_v) {
-  atomicAdd(&t.count[j], 1u);
-  if (!has_v) return;
-  atomicAdd(&t.sum[j], v);
-  if (isnan(v)) return;
+// A row's value into slot j, with g's rows (warp_slot_rows of the warp's slots).
+__device__ __forceinline__ void htab_accum(HTab& t, uint32_t j, const SlotRows& g, double v, bool has_v) {
+  if (g.rows) {
+    atomicAdd(&t.count[j], g.rows);
+    if (__double_as_longlong(g.sum) != 0) atomicAdd(&t.sum[j], g.sum);
+  }
+  if (!has_v || isnan(v)) return;
   const unsigned long long k = f64_ord_key(v);
   const uint32_t w = *reinterpret_cast<volatile uint32_t*>(&t.mm16[j]);
   volatile uint16_t* bound = reinterpret_cast<volatile uint16_t*>(&t.mm16[j]);

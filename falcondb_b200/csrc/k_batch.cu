@@ -76,10 +76,13 @@ __device__ void batch_flush(HTab& tab, const BatchQuery& q, int* err) {
 }
 
 // Bound by latency and by the shared-memory compare-and-swap loops, so resident
-// warps count: three CTAs per SM (40 registers) at one row per thread.  30M rows
-// of 64 Zipf queries over 2000 keys: 0.84 ms; 0.88 at four CTAs (32 registers,
-// spills), 0.92 with two rows per thread, 0.98-1.08 with four (two CTAs), and 1.07
-// with the array-of-structs table at two CTAs.
+// warps count: three CTAs per SM (40 registers) at one row per thread, and whole
+// warps: a row's branches meet again before it is added.  30M rows of 64 Zipf
+// queries over 2000 keys: 0.61 ms; 0.79 without merging a warp's rows, 0.84 when
+// the lanes went on apart after their probes (0.56 and 0.71 for 800 uniform keys).
+// Before those two: 0.88 at four CTAs (32 registers, spills), 0.92 with two rows
+// per thread, 0.98-1.08 with four (two CTAs), and 1.07 with the array-of-structs
+// table at two CTAs.
 __global__ void __launch_bounds__(kBatchThreads, 3) gb_batch_kernel(BatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   HTab& tab = *reinterpret_cast<HTab*>(smem);
@@ -110,23 +113,36 @@ __global__ void __launch_bounds__(kBatchThreads, 3) gb_batch_kernel(BatchArgs a)
     const int64_t* keys = static_cast<const int64_t*>(q.key.values);
     const uint64_t* vals = static_cast<const uint64_t*>(q.val.values);
     const bool f64 = q.val.dtype == FDB_FLOAT64;
-    for (uint64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-      const int64_t key = __ldcs(keys + r);
-      const uint64_t raw = __ldcs(vals + r);
-      const bool has_v = col_valid(q.val, r);
-      const double v = !has_v ? 0.0 : f64 ? __longlong_as_double((long long)raw) : (double)(int64_t)raw;
-      if (!col_valid(q.key, r) || key == INT64_MIN) {  // NULL group
-        htab_accum(tab, kSmemSlots, v, has_v);
-        continue;
+    bool merge = false;  // a tile's rows, by its first
+    for (uint64_t b = r0; b < r1; b += blockDim.x) {
+      const uint64_t r = b + threadIdx.x;
+      int slot = -1;  // the row's CTA slot; -1: none
+      bool has_v = false, spill = false;
+      double v = 0.0;
+      uint64_t skey = 0;
+      if (r < r1) {
+        const int64_t key = __ldcs(keys + r);
+        const uint64_t raw = __ldcs(vals + r);
+        has_v = col_valid(q.val, r);
+        v = !has_v ? 0.0 : f64 ? __longlong_as_double((long long)raw) : (double)(int64_t)raw;
+        if (!col_valid(q.key, r) || key == INT64_MIN) {  // NULL group
+          slot = kSmemSlots;
+        } else {
+          skey = (uint64_t)key ^ (1ull << 63);
+          slot = htab_slot(tab, skey);
+          spill = slot < 0;
+        }
       }
-      const uint64_t skey = (uint64_t)key ^ (1ull << 63);
-      const int slot = htab_slot(tab, skey);
+      if (b == r0) merge = warp_slots_repeat(slot, threadIdx.x & 31);
+      SlotRows g{1u, v};
+      if (merge) g = warp_slot_rows(slot, v, threadIdx.x & 31);
+      __syncwarp();  // or the warp goes on in the pieces that its probes left it in
       if (slot >= 0) {
-        htab_accum(tab, (uint32_t)slot, v, has_v);
-        continue;
+        htab_accum(tab, (uint32_t)slot, g, v, has_v);
+      } else if (spill) {
+        GSlot* dst = gtable_find(q.table, q.mask, skey, a.err);
+        if (dst) gslot_accum(dst, v, has_v);
       }
-      GSlot* dst = gtable_find(q.table, q.mask, skey, a.err);
-      if (dst) gslot_accum(dst, v, has_v);
     }
     __syncthreads();  // the tile is done before s_t is rewritten or the table flushed
   }
