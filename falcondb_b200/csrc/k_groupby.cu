@@ -784,7 +784,7 @@ struct SDTab {
 };
 
 #ifndef FDB_GBD_SLOTS
-#define FDB_GBD_SLOTS 1024
+#define FDB_GBD_SLOTS 2048
 #endif
 constexpr uint32_t kDenseSmemSlots = FDB_GBD_SLOTS;  // power of two
 constexpr int kDenseSmemLog = __builtin_ctz(kDenseSmemSlots);
@@ -803,22 +803,27 @@ constexpr uint32_t kDenseProbe = FDB_GBD_PROBE;
 constexpr uint32_t kDenseSumCopies = FDB_GBD_SUMSPLIT;
 static_assert((kDenseSumCopies & (kDenseSumCopies - 1)) == 0, "SUM copies: a power of two");
 // Launch shape of the two-column instance (key, value): tile rows, stages,
-// consumer warps.
+// consumer warps.  Two CTAs of sixteen warps per SM, one row per thread and tile.
+// What spills goes to the global table in four REDs, so a larger CTA table pays
+// (2048 slots instead of 1024: 40 instead of 45 % of 10M Zipf(1.1) keys' rows
+// spill) as long as a frequent key's rows are merged (warp_slot_rows) and 32 warps
+// stay resident.  Against three CTAs of 1024 slots and eight warps with four rows
+// per thread, GROUP BY in all: 100M rows of 10M Zipf keys 1.72 -> 1.54 ms, 20M of
+// 5000 Zipf keys 0.375 -> 0.305, 60M of 800 uniform keys 0.480 -> 0.445.  Two stages
+// instead of three: 1.60, 0.319, 0.500; 4096 slots in one CTA of 24 warps: 1.93,
+// 0.334, 0.478; 20 warps (registers leave one CTA): 2.08, 0.390, 0.636; merging at
+// the old shape: 1.94, 0.319, 0.511.
 #ifndef FDB_GBD_TR
-#define FDB_GBD_TR 1024
+#define FDB_GBD_TR 512
 #endif
 #ifndef FDB_GBD_ST
-#define FDB_GBD_ST 2
+#define FDB_GBD_ST 3
 #endif
 #ifndef FDB_GBD_NCW
-#define FDB_GBD_NCW 8
+#define FDB_GBD_NCW 16
 #endif
-// Rows a consumer thread decodes together: their tile reads and first CTA
-// table probes are all issued before any of them is applied.
-#ifndef FDB_GBD_ROWS
-#define FDB_GBD_ROWS 4
-#endif
-constexpr uint32_t kDenseRows = FDB_GBD_ROWS;
+// Tiles from one look at whether a warp's rows are worth merging to the next.
+constexpr uint32_t kDenseMergeTiles = 16;
 
 struct GbDenseParams {
   PredProg prog;
@@ -861,12 +866,13 @@ __device__ __forceinline__ SDTab sdtab(unsigned char* sm) {
 // both keys (mmhi, raised after the 64-bit keys): a value whose high half is
 // below the bound cannot improve the slot, so most rows read 8 bytes of the
 // table for MIN and MAX together instead of 16.
-__device__ __forceinline__ void sdslot_accum(const SDTab& t, uint32_t j, double v, bool has_v) {
-  atomicAdd(&t.count[j], 1u);
-  if (!has_v) return;
-  const uint32_t copy = kDenseSumCopies > 1 ? (threadIdx.x & (kDenseSumCopies - 1)) : 0;
-  atomicAdd(&t.sum[copy * (kDenseSmemSlots + 1) + j], v);
-  if (isnan(v)) return;
+__device__ __forceinline__ void sdslot_accum(const SDTab& t, uint32_t j, const SlotRows& g, double v, bool has_v) {
+  if (g.rows) {
+    atomicAdd(&t.count[j], g.rows);
+    const uint32_t copy = kDenseSumCopies > 1 ? (threadIdx.x & (kDenseSumCopies - 1)) : 0;
+    if (__double_as_longlong(g.sum) != 0) atomicAdd(&t.sum[copy * (kDenseSmemSlots + 1) + j], g.sum);
+  }
+  if (!has_v || isnan(v)) return;
   const unsigned long long k = f64_ord_key(v);
 #if FDB_GBD_MMHI
   const unsigned long long w = *reinterpret_cast<volatile unsigned long long*>(&t.mmhi[2 * j]);
@@ -934,76 +940,64 @@ __device__ __forceinline__ int smem_dense_slot_from(const SDTab& t, uint32_t k, 
 
 struct GbDenseOp {
   using Params = GbDenseParams;
-  struct Local {};
+  struct Local {
+    uint32_t tile = 0;
+    bool merge = false;
+  };
   static constexpr size_t kSmem = kDenseSmemBytes;
 
-  static __device__ void init(Local&, const Params&, unsigned char* sm, int ctid, int nct) {
+  static __device__ void init(Local& l, const Params&, unsigned char* sm, int ctid, int nct) {
     uint64_t* w = reinterpret_cast<uint64_t*>(sm);
     for (size_t i = ctid; i < kSmem / 8; i += nct) w[i] = 0;
+    l.tile = 0;
+    l.merge = false;
   }
 
   template <class Acc>
-  static __device__ void step(Local&, const Params& p, unsigned char* sm, const Acc& acc, uint32_t rows, int ctid,
+  static __device__ void step(Local& l, const Params& p, unsigned char* sm, const Acc& acc, uint32_t rows, int ctid,
                               int nct) {
     const SDTab tab = sdtab(sm);
-    constexpr uint32_t R = kDenseRows;
-    enum : uint8_t { kSkip, kNull, kSlot };
-    for (uint32_t i0 = ctid; i0 < rows; i0 += (uint32_t)nct * R) {
-      uint32_t k[R], h[R];
-      unsigned int cur[R];
-      double v[R];
-      uint8_t kind[R];
-      bool has_v[R];
-      // Decode every row first: key, value, its kind and its CTA home slot.
-#pragma unroll
-      for (uint32_t r = 0; r < R; ++r) {
-        const uint32_t i = i0 + r * (uint32_t)nct;
-        kind[r] = kSkip;
-        has_v[r] = false;
-        v[r] = 0.0;
-        k[r] = 0;
-        if (i >= rows) continue;
+    const int lane = ctid & 31;
+    for (uint32_t b = 0; b < rows; b += (uint32_t)nct) {  // whole warps, for the match
+      const uint32_t i = b + ctid;
+      int j = -1;  // the row's CTA slot; -1: none
+      uint32_t k = 0;
+      bool spill = false, has_v = false;
+      double v = 0.0;
+      if (i < rows) {
         const uint64_t row = acc.row(i);
+        bool pass = true;
         if (p.prog.n) {
           GbGetter<Acc> get{p.cols, acc, i, row};
-          if (!eval_prog(p.prog, get)) continue;
+          pass = eval_prog(p.prog, get);
         }
-        const int64_t key = acc.template get<int64_t>(0, i);
-        has_v[r] = p.cols[1].validity ? col_valid(p.cols[1], row) : true;
-        if (has_v[r])
-          v[r] = p.cols[1].dtype == FDB_FLOAT64 ? acc.template get<double>(1, i)
-                                                : (double)acc.template get<int64_t>(1, i);
-        const bool kvalid = (p.cols[0].validity ? col_valid(p.cols[0], row) : true) && key != INT64_MIN;
-        if (!kvalid) {  // NULL group (i64::MIN reads as NULL)
-          kind[r] = kNull;
-          continue;
-        }
-        const uint64_t kk = (uint64_t)key - (uint64_t)p.kmin;
-        if (kk >= p.slots) {  // outside the sized range: the sizing did not see this column
-          atomicExch(p.err, kErrCapacity);
-          continue;
-        }
-        k[r] = (uint32_t)kk;
-        kind[r] = kSlot;
-      }
-      // Every row's first probe in flight together.
-#pragma unroll
-      for (uint32_t r = 0; r < R; ++r) {
-        h[r] = smem_dense_home(k[r]);
-        cur[r] = kind[r] == kSlot ? tab.k1[h[r]] : 0u;
-      }
-#pragma unroll
-      for (uint32_t r = 0; r < R; ++r) {
-        if (kind[r] == kNull) {
-          sdslot_accum(tab, kDenseSmemSlots, v[r], has_v[r]);
-        } else if (kind[r] == kSlot) {
-          const int j = smem_dense_slot_from(tab, k[r], h[r], cur[r]);
-          if (j >= 0)
-            sdslot_accum(tab, (uint32_t)j, v[r], has_v[r]);
-          else
-            dslot_accum(p.table + k[r], v[r], has_v[r]);
+        if (pass) {
+          const int64_t key = acc.template get<int64_t>(0, i);
+          has_v = p.cols[1].validity ? col_valid(p.cols[1], row) : true;
+          if (has_v)
+            v = p.cols[1].dtype == FDB_FLOAT64 ? acc.template get<double>(1, i)
+                                               : (double)acc.template get<int64_t>(1, i);
+          const bool kvalid = (p.cols[0].validity ? col_valid(p.cols[0], row) : true) && key != INT64_MIN;
+          const uint64_t kk = (uint64_t)key - (uint64_t)p.kmin;
+          if (!kvalid) {  // NULL group (i64::MIN reads as NULL)
+            j = (int)kDenseSmemSlots;
+          } else if (kk >= p.slots) {  // outside the sized range: the sizing did not see this column
+            atomicExch(p.err, kErrCapacity);
+          } else {
+            k = (uint32_t)kk;
+            const uint32_t h = smem_dense_home(k);
+            j = smem_dense_slot_from(tab, k, h, tab.k1[h]);
+            spill = j < 0;
+          }
         }
       }
+      if (b == 0 && (l.tile++ & (kDenseMergeTiles - 1)) == 0) l.merge = warp_slots_repeat(j, lane);
+      SlotRows g{1u, v};
+      if (l.merge) g = warp_slot_rows(j, v, lane);
+      if (j >= 0)
+        sdslot_accum(tab, (uint32_t)j, g, v, has_v);
+      else if (spill)
+        dslot_accum(p.table + k, v, has_v);
     }
   }
 
@@ -1796,8 +1790,10 @@ void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& va
     if (n > 0) {
       switch (nc) {
         case 2: launch_stream_gb<GbDenseOp, 2, FDB_GBD_TR, FDB_GBD_ST, FDB_GBD_NCW>(c, all, n, p, GbDenseOp::kSmem); break;
-        case 3: launch_stream_gb<GbDenseOp, 3, 1024, 2, FDB_GBD_NCW>(c, all, n, p, GbDenseOp::kSmem); break;
-        default: launch_stream_gb<GbDenseOp, 4, 512, 3, FDB_GBD_NCW>(c, all, n, p, GbDenseOp::kSmem); break;
+        // Still two CTAs per SM beside the WHERE columns (40M rows, one column:
+        // 800 uniform keys 0.56 ms, 0.74 with tiles of 1024 and one CTA).
+        case 3: launch_stream_gb<GbDenseOp, 3, 512, 2, 16>(c, all, n, p, GbDenseOp::kSmem); break;
+        default: launch_stream_gb<GbDenseOp, 4, 384, 2, 12>(c, all, n, p, GbDenseOp::kSmem); break;
       }
     }
     dense_chunk_count_kernel<<<(unsigned)nchunks, kDenseCompactThreads, 0, c.stream>>>(table, slots, chunk_off);
