@@ -730,17 +730,15 @@ def cpu_baseline(t, n, threads):
 
 
 # ----------------------------------------------------------------------------- secondary workloads
-def radix_bytes_per_row(passes: int, keys_last: bool) -> int:
-    """Algorithmic bytes per row of the radix sort: the key build (read 8,
-    write 12); per digit pass the digit count (the 8-byte keys in the first
-    pass, then the 1-byte digits that the previous scatter wrote), the scatter
-    (read 12; write 12, or only the 4-byte row in a last pass that stores no
-    keys) and, before every pass but the last, the next pass's digit (1)."""
-    b = 20
-    for p in range(passes):
-        last = p == passes - 1
-        b += (8 if p == 0 else 1) + 12 + (12 if keys_last or not last else 4) + (0 if last else 1)
-    return b
+def sort_bytes_per_row(n: int) -> int:
+    """Algorithmic bytes per row of the sample sort, the path of keys that
+    rarely repeat: the first split (read 8, write 12), above 409,600 rows the
+    second (read 12, write 12), and the leaves' read of the pairs (12; one CTA
+    sorts up to 3968 rows straight from the column).  What the leaves write is
+    the caller's to add."""
+    if n <= 3968:
+        return 8
+    return 20 + (24 if n > 409_600 else 0) + 12
 
 
 def _time_steps(fn, K, W, stream, torch):
@@ -946,17 +944,13 @@ def run_secondary(args):
                       "group counts"})
         db.drop_table("g")
     if args.workload in ("sort", "all"):
-        # ORDER BY score DESC over 100M FLOAT64 rows, no LIMIT: an LSD radix
-        # sort of (order key, row) pairs (bytes per row: radix_bytes_per_row).
+        # ORDER BY score DESC over 100M FLOAT64 rows, no LIMIT: a sample sort
+        # of (order key, row) pairs (bytes per row: sort_bytes_per_row, and the
+        # 4-byte row).
         host_sc = W.table_t(n, seed=1)["score"]
         sc = torch.from_numpy(host_sc).to(dev)
         rows_out = torch.empty(n, dtype=torch.int32, device=dev)
         ms = _time_steps(lambda: ops.sort(db, sc, n, True, rows=rows_out), K, Wm, stream, torch)
-        bits = host_sc.view(np.uint64)
-        ordk = np.where(bits >> np.uint64(63) == 0, bits ^ np.uint64(1 << 63), ~bits)  # f64_ord_key
-        vary = int(np.bitwise_or.reduce(ordk)) ^ int(np.bitwise_and.reduce(ordk))
-        passes = sum(1 for byte in range(8) if (vary >> (8 * byte)) & 255)
-        del bits, ordk
         r = rows_out[:n].long()
         s_sorted = sc[r]
         assert bool((s_sorted[1:] <= s_sorted[:-1]).all())
@@ -964,7 +958,7 @@ def run_secondary(args):
         seen[r] = True
         assert bool(seen.all())
         del r, s_sorted, seen
-        nbytes = n * radix_bytes_per_row(passes, keys_last=False)
+        nbytes = n * (sort_bytes_per_row(n) + 4)
         sample = 10_000_000 if n >= 10_000_000 else n
         hs = sc[:sample].cpu().numpy()
         threads = args.cpu_threads or O.hardware_threads()
@@ -972,15 +966,14 @@ def run_secondary(args):
         O.ref_sort(hs, True, threads)
         cpu_s = time.perf_counter() - t0
         line("sort", ms, nbytes, {"rows": n, "query": "SELECT score FROM t ORDER BY score DESC",
-                                  "digit_passes": passes, "mrows_per_s": round(n / (ms / 1e3) / 1e6, 1),
+                                  "mrows_per_s": round(n / (ms / 1e3) / 1e6, 1),
                                   "cpu_sample": {"rows": sample, "mrows_per_s": round(sample / cpu_s / 1e6, 2),
                                                  "cores": threads, "kind": "port",
                                                  "what": "reference-shaped sort: (order key, row) pair loop, "
                                                          "parallel tuple sort (oracle/refengine.cpp ref_sort)"}})
         # SELECT DISTINCT score (first occurrence per value, row order): the same
-        # radix sort on value keys (every pass writes keys), a run-head pass
-        # (read 12 per row, a bit per row of mask) and the mask's compaction
-        # (4 bytes per kept row).
+        # sort on value keys, whose leaves set a bit per kept row in a mask, and
+        # the mask's compaction (4 bytes per kept row).
         dcount = torch.empty(1, dtype=torch.int64, device=dev)
         ms_d = _time_steps(lambda: ops.distinct(db, sc, n, rows=rows_out, count=dcount), K, Wm, stream, torch)
         kept = int(dcount.item())
@@ -989,7 +982,7 @@ def run_secondary(args):
         t0 = time.perf_counter()
         O.distinct(hs_d)
         cpu_d = time.perf_counter() - t0
-        line("distinct", ms_d, n * (radix_bytes_per_row(passes, keys_last=True) + 12) + n // 4 + kept * 4,
+        line("distinct", ms_d, n * sort_bytes_per_row(n) + n // 4 + kept * 4,
              {"rows": n, "query": "SELECT DISTINCT score FROM t", "distinct_values": kept,
               "mrows_per_s": round(n / (ms_d / 1e3) / 1e6, 1),
               "cpu_sample": {"rows": len(hs_d), "mrows_per_s": round(len(hs_d) / cpu_d / 1e6, 2), "cores": 1,
