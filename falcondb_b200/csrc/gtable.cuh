@@ -60,16 +60,6 @@ __device__ __forceinline__ void sslot_accum(GSlot* s, double v, bool has_v) {
   }
 }
 
-// A group of `n` rows folded beforehand: `has_sum` when at least one had a
-// value; nmin / max are 0 when none had a non-NaN value.
-__device__ __forceinline__ void sslot_accum_n(GSlot* s, uint32_t n, bool has_sum, double sum, uint64_t nmin,
-                                              uint64_t max) {
-  atomicAdd(reinterpret_cast<unsigned int*>(&s->count), n);
-  if (has_sum) atomicAdd(&s->sum, sum);
-  if (nmin) atomicMax(&s->nmin, (unsigned long long)nmin);
-  if (max) atomicMax(&s->max, (unsigned long long)max);
-}
-
 __device__ __forceinline__ void gslot_merge(GSlot* s, const GSlot& v) {
   atomicAdd(&s->count, v.count);
   atomicAdd(&s->sum, v.sum);
