@@ -109,21 +109,30 @@ void Ctx::ensure_scratch(size_t bytes) {
   scratch = alloc_buf(want);
 }
 
-bool Ctx::try_scratch(size_t bytes) {
-  if (scratch.bytes >= bytes) return true;
+bool SpareScratch::take(size_t bytes) {
+  if (c_.scratch.bytes >= bytes) return true;
   const size_t want = (bytes + (1u << 20) - 1) & ~size_t((1u << 20) - 1);
-  const size_t others = in_use.load() - scratch.bytes;
-  if (others >= budget || want > (budget - others) / 4) return false;
+  const size_t held = c_.in_use.load();
+  if (taken_ || held >= c_.budget || want > (c_.budget - held) / 4) return false;
   void* p = nullptr;
-  if (cudaMallocAsync(&p, want, stream) != cudaSuccess) {
+  if (cudaMallocAsync(&p, want, c_.stream) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  if (scratch.ptr) free_buf(scratch);
-  scratch.ptr = p;
-  scratch.bytes = want;
-  in_use += want;
+  c_.in_use += want;
+  arena_ = c_.scratch;
+  top_ = c_.scratch_top;
+  c_.scratch.ptr = p;
+  c_.scratch.bytes = want;
+  taken_ = true;
   return true;
+}
+
+SpareScratch::~SpareScratch() {
+  if (!taken_) return;
+  c_.free_buf(c_.scratch);  // in stream order: after the work queued on it
+  c_.scratch = arena_;
+  c_.scratch_top = top_;
 }
 
 void* Ctx::scratch_take(size_t bytes) {
@@ -679,7 +688,6 @@ int fdb_group_by_i64(fdb_db* db, const fdb_dev_column* key, const fdb_dev_column
     CallScope s(db, default_scratch(c));
     const GbSizing sz = group_by_i64_sizing(s.c, *key, nrows, expected_groups);
     s.c.scratch_reset();
-    reserve_group_by_i64(s.c, sz, lf, nrows, nterms);
     op_group_by_i64(s.c, *key, *value, nrows, prog, nterms, pred_cols, npred_cols, sz, lf, d_groups, capacity,
                     d_ngroups);
   });

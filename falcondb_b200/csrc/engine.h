@@ -115,12 +115,29 @@ struct Ctx {
   void* scratch_take(size_t bytes);
   void scratch_reset() { scratch_top = kTicketBytes; }
   void ensure_scratch(size_t bytes);
-  // ensure_scratch for a working buffer that an operator can do without: false,
-  // and nothing changes, when it would take more than a quarter of what the
-  // budget has left or the device has no room for it.
-  bool try_scratch(size_t bytes);
   // Reads and clears d_err (syncs), with what `also` has queued in the same wait.
   int check_device_error(HostReads* also = nullptr);
+};
+
+// A larger scratch arena for one operator call that can do without it: take()
+// puts it in the context's place, and the call's end gives it back, so that
+// nothing of it counts against the budget when the next table, join or arena
+// is allocated.  False, and nothing changes, when it would take more than a
+// quarter of what the budget has left or the device has no room for it.  One
+// object at a time per context, under the context's lock.
+class SpareScratch {
+ public:
+  explicit SpareScratch(Ctx& ctx) : c_(ctx) {}
+  SpareScratch(const SpareScratch&) = delete;
+  SpareScratch& operator=(const SpareScratch&) = delete;
+  ~SpareScratch();
+  bool take(size_t bytes);
+
+ private:
+  Ctx& c_;
+  DevBuf arena_;  // the context's own
+  size_t top_ = 0;
+  bool taken_ = false;
 };
 
 // Copies of device results to the host, queued on the operator stream and
@@ -212,8 +229,7 @@ struct GbSizing {
 // sizing pass over the key column: estimate plus headroom, and the key range
 // (synchronises).
 GbSizing group_by_i64_sizing(Ctx& c, const fdb_dev_column& key, uint64_t n, uint64_t expected_groups);
-// Reserves scratch for op_group_by_i64 of n rows (on top of what is taken).
-void reserve_group_by_i64(Ctx& c, const GbSizing& s, double load_factor, uint64_t n, int nterms);
+// Reserves its own scratch (on top of what is taken).
 void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& value, uint64_t n,
                      const fdb_pred_term* prog, int nterms, const fdb_dev_column* pred_cols,
                      int npred, const GbSizing& s, double load_factor,

@@ -1742,14 +1742,6 @@ static size_t gb_part_scratch(uint64_t n) {
   return n * sizeof(GbRec) + sizeof(GSlot) + (2 * kGbParts + 1) * 4 + 5 * 256;
 }
 
-void reserve_group_by_i64(Ctx& c, const GbSizing& s, double load_factor, uint64_t n, int nterms) {
-  const size_t tables = group_by_i64_scratch(s, load_factor) + (16u << 20);
-  if (gb_partitions(s, load_factor, n, nterms) &&
-      c.try_scratch(c.scratch_top + std::max(tables, gb_part_scratch(n) + (1u << 20))))
-    return;
-  c.ensure_scratch(tables);
-}
-
 void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& value, uint64_t n,
                      const fdb_pred_term* prog, int nterms, const fdb_dev_column* pred_cols,
                      int npred, const GbSizing& sz, double load_factor,
@@ -1771,6 +1763,11 @@ void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& va
     if (!all[i].values && n > 0) fail(FDB_E_ARG, "column without values");
     dcols[i] = DevCol{all[i].dtype, all[i].values, all[i].validity, all[i].validity_offset};
   }
+
+  SpareScratch spare(c);
+  const bool parts =
+      gb_partitions(sz, load_factor, n, nterms) && spare.take(c.scratch_top + gb_part_scratch(n));
+  if (!parts) c.ensure_scratch(group_by_i64_scratch(sz, load_factor) + (16u << 20));
 
   if (const uint64_t slots = gb_dense_slots(sz, load_factor)) {
     // Direct-addressed table: slot k - kmin per key value, NULL group after it.
@@ -1807,7 +1804,7 @@ void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& va
     return;
   }
 
-  if (gb_partitions(sz, load_factor, n, nterms) && c.scratch_top + gb_part_scratch(n) <= c.scratch.bytes) {
+  if (parts) {
     GbRec* rec = static_cast<GbRec*>(c.scratch_take(n * sizeof(GbRec)));
     GSlot* null_slot = static_cast<GSlot*>(c.scratch_take(sizeof(GSlot)));
     uint32_t* off = static_cast<uint32_t*>(c.scratch_take((kGbParts + 1) * 4));

@@ -721,15 +721,15 @@ static MsdPlan msd_plan(uint64_t m) {
 }
 
 // Reserves scratch for a sort of up to n pairs beyond `base` bytes: the sample
-// sort's when the arena may grow that far (twice the radix passes' need),
-// otherwise the radix passes' alone.
-static void reserve_sort(Ctx& c, uint64_t n, size_t base, bool nullable) {
+// sort's (twice the radix passes' need) from `spare` when that may be taken,
+// otherwise the radix passes' alone from the arena.
+static void reserve_sort(Ctx& c, SpareScratch& spare, uint64_t n, size_t base, bool nullable) {
   const size_t radix = c.scratch_top + base + sort_scratch_bytes(n, nullable);
   if (n > kMsdLeafCap && n <= kMsdTwoLevels) {
     // A NULL split leaves fewer pairs, whose plan is no larger but for rounding.
     const size_t split = nullable ? (n + 63) / 64 * 8 + 2 * n * 4 + (2u << 20) : 0;
     const size_t msd = c.scratch_top + base + split + msd_plan(n).bytes;
-    if (c.try_scratch(std::max(radix, msd) + (1u << 20))) return;
+    if (spare.take(std::max(radix, msd) + (1u << 20))) return;
   }
   c.ensure_scratch(radix);
 }
@@ -941,9 +941,8 @@ void op_sort_keyed(Ctx& c, const fdb_dev_column& col, uint64_t n, bool desc, boo
   if (!col.values) fail(FDB_E_ARG, "column without values");
   const DevCol dc{col.dtype, col.values, col.validity, col.validity_offset};
   set_scatter_smem();
-  // Working memory comes from the context's scratch arena, which grows once
-  // and stays resident.
-  reserve_sort(c, n, 0, col.validity != nullptr);
+  SpareScratch spare(c);
+  reserve_sort(c, spare, n, 0, col.validity != nullptr);
 
   // NULL rows leave the sort: the valid rows are sorted, the NULL rows keep
   // their row order before or after them.
@@ -992,7 +991,8 @@ void op_distinct(Ctx& c, const fdb_dev_column& col, uint64_t n, uint32_t* d_rows
   const DevCol dc{col.dtype, col.values, col.validity, col.validity_offset};
   set_scatter_smem();
   const uint64_t words = (n + 63) / 64;
-  reserve_sort(c, n, words * 8 + 256, col.validity != nullptr);
+  SpareScratch spare(c);
+  reserve_sort(c, spare, n, words * 8 + 256, col.validity != nullptr);
   unsigned long long* heads = static_cast<unsigned long long*>(c.scratch_take(words * 8));
   FDB_CUDA(cudaMemsetAsync(heads, 0, words * 8, c.stream));
 

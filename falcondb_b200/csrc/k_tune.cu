@@ -110,7 +110,6 @@ void run_kind(Ctx& c, int kind, const Synth& s, uint64_t n, HashTable* ht) {
       sz.kmin = 0;
       sz.kmax = (int64_t)groups - 1;
       c.scratch_reset();
-      reserve_group_by_i64(c, sz, 0.5, n, 0);
       op_group_by_i64(c, gkey, score, n, nullptr, 0, nullptr, 0, sz, 0.5,
                       reinterpret_cast<fdb_group_i64*>(out + 8192), groups + 2, reinterpret_cast<uint64_t*>(out));
       break;

@@ -1082,7 +1082,6 @@ static void run_aggregates(Plan& plan, const Rel& rel, const Query& q, fdb_resul
       plan.c.scratch_reset();
       const GbSizing sz = group_by_i64_sizing(plan.c, col.dev, rel.nrows, 0);
       plan.c.scratch_reset();
-      reserve_group_by_i64(plan.c, sz, 0.5, rel.nrows, (int)prog.size());
       op_group_by_i64(plan.c, col.dev, col.dev, rel.nrows, prog.data(), (int)prog.size(), pcols.data(),
                       (int)pcols.size(), sz, 0.5, d, cap, dn);
       const uint64_t ng = plan.checked_one(dn);
@@ -1228,7 +1227,6 @@ static void run_group_by(Plan& plan, const Rel& rel, const Query& q, fdb_result*
     std::vector<fdb_group_i64> groups;
     if (rel.nrows > 0) {
       const GbSizing sz = group_by_i64_sizing(plan.c, key.dev, rel.nrows, 0);
-      reserve_group_by_i64(plan.c, sz, 0.5, rel.nrows, (int)prog.size());
       op_group_by_i64(plan.c, key.dev, rel.cols[vc].dev, rel.nrows, prog.data(), (int)prog.size(), pcols.data(),
                       (int)pcols.size(), sz, 0.5, d, cap, dn);
       groups = plan.to_host(d, plan.checked_one(dn));
