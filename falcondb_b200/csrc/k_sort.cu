@@ -678,6 +678,7 @@ struct MsdPlan {
   uint32_t samples = 0;
   uint32_t parts1 = 0, cap1 = 0;
   uint32_t parts2 = 0, cap2 = 0;  // parts2 = 0: one level, whose buckets are the leaves
+  uint32_t spill = 0;             // pairs of leaves that overflow, when there are two
   size_t bytes = 0;
 };
 
@@ -705,18 +706,18 @@ static MsdPlan msd_plan(uint64_t m) {
     p.cap1 = (uint32_t)((m / kMsdFirst * 23 / 10 + 319) / 64 * 64);
     p.parts2 = pow2((m + kMsdFirst * kMsdLeafRows - 1) / (kMsdFirst * kMsdLeafRows));
     p.cap2 = leaf_cap(m / ((uint64_t)kMsdFirst * p.parts2));
+    p.spill = (uint32_t)(m / 16);
   }
   // A leaf's size varies with the shares that both levels' samples give it.  With
   // 32 samples per first-level bucket some bucket of 256 is 1.7 times the average,
   // and where a leaf has few samples of its own (64 from 128 parts on) one in 10 to
-  // 100 sorts of 100M keys then overflowed a leaf, at the price of a radix sort
-  // (9.5 ms instead of 2.5).  With twice the samples there (1.4 times) a leaf's
+  // 100 sorts of 100M keys then overflowed a leaf.  With twice the samples there (1.4 times) a leaf's
   // capacity is seven of its standard deviations away.
   p.samples = p.parts2 >= 64 ? 2048 * kMsdSampleItems : m >= 1024 * kMsdSampleItems ? 1024 * kMsdSampleItems : 2048;
   const uint64_t leaves = (uint64_t)p.parts1 * std::max(1u, p.parts2);
   // Pairs of both levels, the maps, counters and offsets, and 256-byte rounding.
-  p.bytes = (size_t)p.parts1 * p.cap1 * 12 + (size_t)p.parts1 * p.parts2 * p.cap2 * 12 + leaves * 44 +
-            (p.parts1 + 1) * (sizeof(MsdMap) + 16) + 16 * 256;
+  p.bytes = (size_t)p.parts1 * p.cap1 * 12 + (size_t)p.parts1 * p.parts2 * p.cap2 * 12 + (size_t)p.spill * 12 +
+            leaves * 44 + (p.parts1 + 1) * (sizeof(MsdMap) + 16) + 18 * 256;
   return p;
 }
 
@@ -812,33 +813,44 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
     return false;
   }
   c.scratch_top = mark;
-  uint64_t* k1 = static_cast<uint64_t*>(c.scratch_take(n1 * 8));
-  uint32_t* v1 = static_cast<uint32_t*>(c.scratch_take(n1 * 4));
   MsdLeaf* leaf = static_cast<MsdLeaf*>(c.scratch_take(leaves * sizeof(MsdLeaf)));
   uint32_t* big = static_cast<uint32_t*>(c.scratch_take(leaves * 4));
+  uint64_t* k2 = nullptr;
+  uint32_t *v2 = nullptr, *first = nullptr;
+  MsdMap* map2 = nullptr;
+  MsdSpill spill{nullptr, nullptr, p.spill};
+  if (p.parts2) {
+    k2 = static_cast<uint64_t*>(c.scratch_take(leaves * p.cap2 * 8));
+    v2 = static_cast<uint32_t*>(c.scratch_take(leaves * p.cap2 * 4));
+    map2 = static_cast<MsdMap*>(c.scratch_take(p.parts1 * sizeof(MsdMap)));
+    first = static_cast<uint32_t*>(c.scratch_take((p.parts1 + 1) * 4));
+    spill.keys = static_cast<uint64_t*>(c.scratch_take((size_t)p.spill * 8));
+    spill.pos = static_cast<uint32_t*>(c.scratch_take((size_t)p.spill * 4));
+  }
+  // The first level's pairs lie last: their room is free for the leaves that
+  // overflow once the second level has them.
+  const size_t level1 = c.scratch_top;
+  uint64_t* k1 = static_cast<uint64_t*>(c.scratch_take(n1 * 8));
+  uint32_t* v1 = static_cast<uint32_t*>(c.scratch_take(n1 * 4));
   const uint32_t tiles = (m + kMsdTile - 1) / kMsdTile;
   msd_split_kernel<Src, false><<<tiles, kMsdThreads, sizeof(MsdSplitSmem), c.stream>>>(
-      src, m, nullptr, nullptr, nullptr, 0, nullptr, 0, map1, p.parts1, p.cap1, k1, v1, cur1, state);
+      src, m, nullptr, nullptr, nullptr, 0, nullptr, 0, map1, p.parts1, p.cap1, k1, v1, cur1, MsdSpill{}, state);
   const uint64_t* lk = k1;
   const uint32_t* lv = v1;
   uint32_t lcap = p.cap1;
   if (p.parts2) {
-    uint64_t* k2 = static_cast<uint64_t*>(c.scratch_take(leaves * p.cap2 * 8));
-    uint32_t* v2 = static_cast<uint32_t*>(c.scratch_take(leaves * p.cap2 * 4));
-    MsdMap* map2 = static_cast<MsdMap*>(c.scratch_take(p.parts1 * sizeof(MsdMap)));
-    uint32_t* first = static_cast<uint32_t*>(c.scratch_take((p.parts1 + 1) * 4));
     if (p.parts2 <= 128)
-      msd_subsample_kernel<8><<<p.parts1, 1024, 0, c.stream>>>(k1, cur1, p.cap1, p.parts2, map2, first, state);
+      msd_subsample_kernel<8><<<p.parts1, 1024, 0, c.stream>>>(k1, cur1, p.cap1, p.parts2, p.spill, map2, first, state);
     else
-      msd_subsample_kernel<16><<<p.parts1, 1024, 0, c.stream>>>(k1, cur1, p.cap1, p.parts2, map2, first, state);
+      msd_subsample_kernel<16><<<p.parts1, 1024, 0, c.stream>>>(k1, cur1, p.cap1, p.parts2, p.spill, map2, first, state);
     msd_split_kernel<Src, true><<<tiles + p.parts1, kMsdThreads, sizeof(MsdSplitSmem), c.stream>>>(
-        src, m, k1, v1, cur1, p.cap1, first, p.parts1, map2, p.parts2, p.cap2, k2, v2, cur2, state);
-    msd_leaves_kernel<<<p.parts1, kMsdThreads, 0, c.stream>>>(cur1, cur2, map2, p.parts2, leaf, big, state);
+        src, m, k1, v1, cur1, p.cap1, first, p.parts1, map2, p.parts2, p.cap2, k2, v2, cur2, spill, state);
+    msd_leaves_kernel<<<p.parts1, kMsdThreads, 0, c.stream>>>(cur1, cur2, p.cap2, map2, p.parts2, leaf, big, state);
     lk = k2;
     lv = v2;
     lcap = p.cap2;
   } else {
-    msd_leaves_kernel<<<1, kMsdThreads, 0, c.stream>>>(cur1, cur1, map1, p.parts1, leaf, big, state);
+    msd_leaves_kernel<<<1, kMsdThreads, 0, c.stream>>>(cur1, cur1, p.cap1, map1, p.parts1, leaf, big, state);
   }
   const unsigned gbig = (unsigned)std::min<uint64_t>(leaves, 4ull * c.sm_count);
   if (heads) {
@@ -853,8 +865,36 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
                                                                                         nullptr, state);
   }
   read_states();
+  bool done = !(host[kMsdOverflow1] | host[kMsdUneven2] | host[kMsdOverflow2]);
+  if (done && host[kMsdOverLeaves]) {
+    // Leaves that overflowed: their pairs, spilled or in their (full) regions,
+    // sorted by position, then by key.
+    const uint32_t nover = host[kMsdOverLeaves];
+    const uint64_t n = host[kMsdSpilled] + (uint64_t)nover * p.cap2;
+    done = n <= p.spill;
+    if (done) {
+      const uint32_t* over = big + leaves - 1;
+      c.scratch_top = level1;
+      msd_over_collect_kernel<<<nover, 256, 0, c.stream>>>(k2, v2, p.cap2, over, spill, state);
+      const unsigned g = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)c.sm_count * 8);
+      const uint64_t* sk = nullptr;
+      const uint32_t *order = nullptr, *sv = nullptr;
+      auto keys_of = [&](uint64_t* k, uint32_t* v, unsigned long long* vary, const uint32_t*) {
+        msd_over_keys_kernel<<<g, 256, 0, c.stream>>>(spill, order, (uint32_t)n, k, v, vary);
+      };
+      const uint32_t* by_pos = nullptr;
+      radix_sort_pairs(c, (uint32_t)n, keys_of, nullptr, &sk, &by_pos);
+      order = by_pos;
+      radix_sort_pairs(c, (uint32_t)n, keys_of, nullptr, &sk, &sv);
+      if (heads)
+        msd_over_write_kernel<Src, true><<<nover, 256, 0, c.stream>>>(src, over, nover, leaf, sk, sv, nullptr, heads);
+      else
+        msd_over_write_kernel<Src, false><<<nover, 256, 0, c.stream>>>(src, over, nover, leaf, sk, sv, rows, nullptr);
+      FDB_CUDA(cudaGetLastError());
+    }
+  }
   c.scratch_top = mark;
-  return !(host[kMsdOverflow1] | host[kMsdUneven2] | host[kMsdOverflow2]);
+  return done;
 }
 
 template <int DT, int MODE, class KeysFn>

@@ -23,9 +23,16 @@
 //                       bucket whose keys crowd into few slots is sorted by a
 //                       bitonic network instead.
 //
-// (100M float64 keys: the times are in k_sort.cu.)  A bucket that overflows its region, or a map
-// whose steps cannot split the keys evenly, sets the state word of its level; the
-// kernels after it return at once and the caller runs the radix passes instead.
+//   msd_over_*_kernel   leaves of two-level sorts that hold more pairs than their
+//                       region: what the region has no room for is spilled to a
+//                       list, the region's pairs join it, and the list (a few per
+//                       cent of the pairs) is sorted by radix passes.  These are
+//                       values with some 2400 to 40,000 of 100M rows, too few for
+//                       the sample to see, and other clusters of close keys.
+//
+// A first-level bucket that overflows its region, or more spilled pairs than the
+// list takes, sets a state word; the kernels after it return at once and the
+// caller runs the radix passes instead.
 #pragma once
 #include <type_traits>
 
@@ -52,11 +59,13 @@ static_assert(kMsdSlots == 16 * kMsdLeafThreads, "a thread's slots are two 16-by
 static_assert(kMsdLeafCap <= kMsdLeafThreads * kMsdBigItems, "a leaf fits its threads' items");
 
 // State words, nonzero when the sort stopped: set by the sample, by a
-// first-level overflow, by the second-level samples, by a second-level
-// overflow.  A kernel reads only the words that kernels before it write, so all
-// its threads see the same.
+// first-level overflow, by the second-level samples, by more spilled pairs than
+// there is room for.  A kernel reads only the words that kernels before it write,
+// so all its threads see the same.
 constexpr int kMsdRepeats = 0, kMsdOverflow1 = 1, kMsdUneven2 = 2, kMsdOverflow2 = 3, kMsdStates = 4;
-constexpr int kMsdBigCount = 8;  // state[8]: leaves of more than kMsdLeafMost pairs
+// Counters: leaves of more than kMsdLeafMost pairs; pairs that their leaf's region
+// had no room for, and those leaves; pairs in steps that nearly fill a leaf.
+constexpr int kMsdBigCount = 8, kMsdSpilled = 9, kMsdOverLeaves = 10, kMsdUnevenPairs = 11;
 
 __device__ __forceinline__ bool msd_stopped(const uint32_t* state, int words) {
   uint32_t x = 0;
@@ -270,13 +279,15 @@ __device__ __forceinline__ uint32_t msd_build_map(MsdMapSmem& S, const uint64_t 
   return S.heaviest;
 }
 
-// One CTA.  The sort stops, for the radix passes, when at most `few_bytes` bytes
-// of the sampled keys vary, when some key's sampled share means more than about
-// 1024 pairs of it (`run` + 1 equal samples), when equal samples are so many that
-// most keys have 16 pairs or more (8 samples^2 / m: keys of r pairs each give
-// samples^2 r / 2m), or when one step of the map holds far more than a bucket.
-// The first eighth of the samples is looked at by itself, so that clear cases
-// stop after one round trip to memory.
+// The sort stops, for the radix passes, when at most `few_bytes` bytes of the
+// sampled keys vary, when some key has `run` + 1 equal samples (a sampled share of
+// about 1024 pairs, but at least four samples: 49,000 of 100M pairs), when equal
+// samples are so many that most keys have 16 pairs or more (8 samples^2 / m: keys
+// of r pairs each give samples^2 r / 2m), or when one step of the map holds far
+// more than a bucket.  K keys of r pairs among others that do not repeat go unseen
+// up to about K r^2 = 2.8e9 (m / 1e8)^2, which is 1.2 % of 100M pairs at r = 2400
+// and fewer above: what spills.  The first eighth of the samples is looked at by
+// itself, so that clear cases stop after one round trip to memory.
 constexpr uint32_t kMsdSeen = 2 * 1024 * kMsdSampleItems;  // hash slots of the equal-sample check
 struct MsdSampleSmem {
   MsdMapSmem map;
@@ -288,8 +299,7 @@ struct MsdSampleSmem {
 };
 static_assert(kMsdSeen == 1u << 14, "hash bits of the equal-sample check");
 
-//
-// kItems samples per thread: the equal-sample check takes the first
+// One CTA, kItems samples per thread: the equal-sample check takes the first
 // kMsdSampleItems of them, the map all.
 template <class Src, int kItems>
 __global__ void __launch_bounds__(1024) msd_sample_kernel(Src src, uint32_t m, int log_samples, uint32_t parts,
@@ -364,8 +374,8 @@ __global__ void __launch_bounds__(1024) msd_sample_kernel(Src src, uint32_t m, i
 // before each one have (first[b], b <= gridDim.x).
 template <int kItems>
 __global__ void __launch_bounds__(1024) msd_subsample_kernel(const uint64_t* keys, const uint32_t* cursor, uint32_t cap,
-                                                             uint32_t parts, MsdMap* maps, uint32_t* first,
-                                                             uint32_t* state) {
+                                                             uint32_t parts, uint32_t spill_cap, MsdMap* maps,
+                                                             uint32_t* first, uint32_t* state) {
   __shared__ MsdMapSmem S;
   if (msd_stopped(state, kMsdOverflow1 + 1)) return;
   const uint32_t tid = threadIdx.x;
@@ -397,8 +407,10 @@ __global__ void __launch_bounds__(1024) msd_subsample_kernel(const uint64_t* key
     k[i] = tid < per ? src[msd_sample_pos(tid * kItems + i, log_samples, n)] : 0;
   }
   const uint32_t fullest = msd_build_map(S, k, per, log_samples, parts, maps + blockIdx.x);
-  // A step that alone nearly fills a leaf (small buckets never do).
-  if (tid == 0 && (((uint64_t)fullest * n) >> log_samples) > kMsdLeafCap * 3 / 4) state[kMsdUneven2] = 1;
+  // A step that alone nearly fills a leaf (small buckets never do) will spill.
+  const uint32_t pairs = (uint32_t)(((uint64_t)fullest * n) >> log_samples);
+  if (tid == 0 && pairs > kMsdLeafCap * 3 / 4 && atomicAdd(&state[kMsdUnevenPairs], pairs) + pairs > spill_cap)
+    state[kMsdUneven2] = 1;
 }
 
 struct MsdSplitSmem {
@@ -416,16 +428,23 @@ struct MsdSplitSmem {
 // (kSecond false): tile blockIdx.x of the source, buckets 0 .. parts - 1.
 // Second level: the tiles of the first level's buckets (kin, vin, in_count,
 // in_cap, first), bucket b's parts being buckets b * parts ...  Bucket x's
-// pairs go to kout / vout [x * cap, ...), counted in cursor[x].  Bound by
+// pairs go to kout / vout [x * cap, ...), counted in cursor[x].  Second-level
+// pairs beyond their region go to the spill list.  Bound by
 // shared memory (a table read, one atomic and two or three stores at random
 // places per pair: the LSU data pipe is 72 % busy) and by the write of short
 // runs; 0.68 and 0.84 ms for 100M pairs, 2.9 TB/s.
+struct MsdSpill {
+  uint64_t* keys;
+  uint32_t* pos;
+  uint32_t cap;
+};
 template <class Src, bool kSecond>
 __global__ void __launch_bounds__(kMsdThreads, 3)
     msd_split_kernel(Src src, uint32_t m, const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                      const uint32_t* __restrict__ in_count, uint32_t in_cap, const uint32_t* __restrict__ first,
                      uint32_t nfirst, const MsdMap* __restrict__ maps, uint32_t parts, uint32_t cap,
-                     uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t* cursor, uint32_t* state) {
+                     uint64_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t* cursor, MsdSpill spill,
+                     uint32_t* state) {
   extern __shared__ __align__(128) unsigned char msd_smem[];
   MsdSplitSmem& S = *reinterpret_cast<MsdSplitSmem*>(msd_smem);
   if (msd_stopped(state, kSecond ? kMsdUneven2 + 1 : kMsdRepeats + 1)) return;
@@ -487,7 +506,7 @@ __global__ void __launch_bounds__(kMsdThreads, 3)
   const uint32_t s = msd_block_scan<kMsdThreads>(c, S.scan);
   if (tid < parts) {
     S.start[tid] = s;
-    if (g + c > cap) atomicExch(state + (kSecond ? kMsdOverflow2 : kMsdOverflow1), 1u);
+    if (!kSecond && g + c > cap) atomicExch(state + kMsdOverflow1, 1u);
     S.base[tid] = g - s;
   }
   __syncthreads();
@@ -515,16 +534,30 @@ __global__ void __launch_bounds__(kMsdThreads, 3)
         const size_t at = (size_t)(bucket * parts + x) * cap + o;
         kout[at] = S.keys[p];
         vout[at] = kSecond ? w : t0 + (w & 0xFFFFu);
+      } else if (kSecond) {
+        const unsigned act = __activemask();  // one atomic for the lanes that are here
+        const int lane = tid & 31, first_lane = __ffs(act) - 1;
+        uint32_t q = 0;
+        if (lane == first_lane) q = atomicAdd(state + kMsdSpilled, (uint32_t)__popc(act));
+        q = __shfl_sync(act, q, first_lane) + __popc(act & ((1u << lane) - 1u));
+        if (q < spill.cap) {
+          spill.keys[q] = S.keys[p];
+          spill.pos[q] = w;
+        } else {
+          atomicExch(state + kMsdOverflow2, 1u);
+        }
       }
     }
   }
 }
 
 // Describes the leaves: CTA b those of first-level bucket b (`parts` of them, of
-// map b); with one level, CTA 0 all.  above[] counts the buckets' pairs.
+// map b); with one level, CTA 0 all.  above[] counts the buckets' pairs.  Lists
+// the big leaves from big[0] on, and those with more pairs than their region
+// (`cap`) from big[leaves - 1] down.
 __global__ void __launch_bounds__(kMsdThreads) msd_leaves_kernel(const uint32_t* above, const uint32_t* count,
-                                                                 const MsdMap* maps, uint32_t parts, MsdLeaf* leaves,
-                                                                 uint32_t* big, uint32_t* state) {
+                                                                 uint32_t cap, const MsdMap* maps, uint32_t parts,
+                                                                 MsdLeaf* leaves, uint32_t* big, uint32_t* state) {
   __shared__ uint32_t sm[32];
   __shared__ uint32_t before;
   if (msd_stopped(state, kMsdStates)) return;
@@ -553,7 +586,10 @@ __global__ void __launch_bounds__(kMsdThreads) msd_leaves_kernel(const uint32_t*
     }
   }
   leaves[blockIdx.x * parts + tid] = l;
-  if (c > kMsdLeafMost) big[atomicAdd(state + kMsdBigCount, 1u)] = blockIdx.x * parts + tid;
+  if (c > cap)
+    big[gridDim.x * parts - 1 - atomicAdd(state + kMsdOverLeaves, 1u)] = blockIdx.x * parts + tid;
+  else if (c > kMsdLeafMost)
+    big[atomicAdd(state + kMsdBigCount, 1u)] = blockIdx.x * parts + tid;
 }
 
 template <int kItems>
@@ -768,7 +804,7 @@ __global__ void __launch_bounds__(kMsdLeafThreads, 5)
   extern __shared__ __align__(128) unsigned char msd_smem[];
   if (msd_stopped(state, kMsdStates)) return;
   const MsdLeaf l = leaves[blockIdx.x];
-  if (l.count == 0 || l.count > kMsdLeafMost) return;
+  if (l.count == 0 || l.count > min(kMsdLeafMost, cap)) return;
   const size_t in0 = (size_t)blockIdx.x * cap;
   msd_leaf<Src, kHeads, false, kMsdLeafItems>(src, l, keys + in0, pos + in0, rows, mask,
                                               *reinterpret_cast<MsdLeafSmem<kMsdLeafItems>*>(msd_smem));
@@ -797,6 +833,84 @@ __global__ void __launch_bounds__(kMsdLeafThreads, 4)
       msd_leaf<Src, kHeads, false, kMsdBigItems>(src, l, keys + in0, pos + in0, rows, mask, S);
       __syncthreads();
     }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The leaves with more pairs than their region: over[0], over[-1], ...  100M rows
+// with ten values of 5000 rows, or a hundred: 2.85 and 2.92 ms in all (8.69 and
+// 8.67 when one such leaf sent every row to the radix passes, which alone take
+// 7.8); 30M with ten 1.26 ms (2.90).
+// ---------------------------------------------------------------------------
+
+// CTA b adds the region of the b-th of them to the spill list.
+__global__ void __launch_bounds__(256) msd_over_collect_kernel(const uint64_t* __restrict__ keys,
+                                                               const uint32_t* __restrict__ pos, uint32_t cap,
+                                                               const uint32_t* over, MsdSpill spill, uint32_t* state) {
+  __shared__ uint32_t base;
+  if (threadIdx.x == 0) base = atomicAdd(state + kMsdSpilled, cap);
+  __syncthreads();
+  const size_t in0 = (size_t)over[-(ptrdiff_t)blockIdx.x] * cap;
+  for (uint32_t i = threadIdx.x; i < cap; i += blockDim.x)
+    if (base + i < spill.cap) {
+      spill.keys[base + i] = keys[in0 + i];
+      spill.pos[base + i] = pos[in0 + i];
+    }
+}
+
+// Radix pairs of the n listed pairs: (position, index) without `order`, then, in
+// the order that these sorted to, (key, position): radix passes are stable, so
+// equal keys end up by position.  What varies as the other key kernels have it.
+__global__ void __launch_bounds__(256) msd_over_keys_kernel(MsdSpill spill, const uint32_t* __restrict__ order,
+                                                            uint32_t n, uint64_t* __restrict__ keys,
+                                                            uint32_t* __restrict__ vals, unsigned long long* vary) {
+  unsigned long long o = 0, a = ~0ull;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t at = order ? order[i] : i;
+    const uint64_t k = order ? spill.keys[at] : spill.pos[at];
+    keys[i] = k;
+    vals[i] = order ? spill.pos[at] : i;
+    o |= k;
+    a &= k;
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    o |= __shfl_xor_sync(0xffffffffu, o, s);
+    a &= __shfl_xor_sync(0xffffffffu, a, s);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicOr(&vary[0], o);
+    atomicOr(&vary[1], ~a);
+  }
+}
+
+// CTA b writes the b-th leaf's part of the sorted list, as msd_leaf would: leaves
+// follow one another in key order, so it starts after the pairs of the listed
+// leaves of smaller number.
+template <class Src, bool kHeads>
+__global__ void __launch_bounds__(256) msd_over_write_kernel(Src src, const uint32_t* over, uint32_t nover,
+                                                             const MsdLeaf* __restrict__ leaves,
+                                                             const uint64_t* __restrict__ keys,
+                                                             const uint32_t* __restrict__ pos,
+                                                             uint32_t* __restrict__ rows, unsigned long long* mask) {
+  __shared__ uint32_t start;
+  const uint32_t leaf = over[-(ptrdiff_t)blockIdx.x];
+  if (threadIdx.x == 0) start = 0;
+  __syncthreads();
+  uint32_t before = 0;
+  for (uint32_t j = threadIdx.x; j < nover; j += blockDim.x) {
+    const uint32_t other = over[-(ptrdiff_t)j];
+    if (other < leaf) before += leaves[other].count;
+  }
+  if (before) atomicAdd(&start, before);
+  __syncthreads();
+  const uint32_t n = leaves[leaf].count, out0 = leaves[leaf].out, in0 = start;
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    const uint32_t row = src.row(pos[in0 + i]);
+    if (!kHeads)
+      rows[out0 + i] = row;
+    else if (i == 0 || keys[in0 + i] != keys[in0 + i - 1])
+      atomicOr(&mask[row >> 6], 1ull << (row & 63));
   }
 }
 
