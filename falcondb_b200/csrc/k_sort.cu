@@ -758,17 +758,18 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
     set((const void*)msd_leaf_kernel<Src, true>, sizeof(MsdLeafSmem<kMsdLeafItems>));
     set((const void*)msd_big_leaf_kernel<Src, false, false>, sizeof(MsdLeafSmem<kMsdBigItems>));
     set((const void*)msd_big_leaf_kernel<Src, true, false>, sizeof(MsdLeafSmem<kMsdBigItems>));
-    set((const void*)msd_big_leaf_kernel<Src, false, true>, sizeof(MsdLeafSmem<kMsdBigItems>));
-    set((const void*)msd_big_leaf_kernel<Src, true, true>, sizeof(MsdLeafSmem<kMsdBigItems>));
+    set((const void*)msd_big_leaf_kernel<Src, false, true>, sizeof(MsdDirectSmem));
+    set((const void*)msd_big_leaf_kernel<Src, true, true>, sizeof(MsdDirectSmem));
   });
   constexpr size_t kSmall = sizeof(MsdLeafSmem<kMsdLeafItems>), kBig = sizeof(MsdLeafSmem<kMsdBigItems>);
   if (m <= kMsdLeafCap) {
+    constexpr size_t kDirect = sizeof(MsdDirectSmem);
     if (heads)
-      msd_big_leaf_kernel<Src, true, true><<<1, kMsdLeafThreads, kBig, c.stream>>>(src, m, nullptr, nullptr, nullptr,
-                                                                                  nullptr, 0, nullptr, heads, nullptr);
+      msd_big_leaf_kernel<Src, true, true><<<1, kMsdLeafThreads, kDirect, c.stream>>>(
+          src, m, nullptr, nullptr, nullptr, nullptr, 0, nullptr, heads, nullptr);
     else
-      msd_big_leaf_kernel<Src, false, true><<<1, kMsdLeafThreads, kBig, c.stream>>>(src, m, nullptr, nullptr, nullptr,
-                                                                                   nullptr, 0, rows, nullptr, nullptr);
+      msd_big_leaf_kernel<Src, false, true><<<1, kMsdLeafThreads, kDirect, c.stream>>>(
+          src, m, nullptr, nullptr, nullptr, nullptr, 0, rows, nullptr, nullptr);
     FDB_CUDA(cudaGetLastError());
     return true;
   }
