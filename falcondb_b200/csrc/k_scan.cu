@@ -1090,10 +1090,12 @@ __global__ void compact_scan_kernel(uint64_t* counts, uint64_t nchunks, uint64_t
 // takes one 32-row half word per store, so its lanes write neighbouring
 // entries.  (A thread writing its own words' rows one by one stored 22 separate
 // sectors per warp instruction: 81 us for 10M of 40M rows, 31 us now.)  A chunk
-// with at most one row in 16 passing is listed in shared memory by each word's
+// with at most one row in four passing is listed in shared memory by each word's
 // own thread instead and then copied out: walking its words costs more than
-// its rows.
-constexpr uint32_t kSparseRows = kChunkWords * 64 / 16;
+// its rows (60M rows, the whole call: 7 % 45.5 us listed, 73.6 by words, 59.7 with
+// the threads' own stores; 20 % 56.5, 74.2, 105; a list for more rows than that
+// would take the shared memory of the CTAs beside it).
+constexpr uint32_t kSparseRows = kChunkWords * 64 / 4;
 __global__ void __launch_bounds__(kCompactThreads)
     compact_write_kernel(const uint64_t* mask, uint64_t nwords, const uint64_t* offsets, uint32_t* rows,
                          uint64_t capacity) {
