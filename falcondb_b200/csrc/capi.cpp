@@ -686,7 +686,7 @@ int fdb_group_by_i64(fdb_db* db, const fdb_dev_column* key, const fdb_dev_column
     Ctx& c = db->ctx;
     double lf = (load_factor > 0.0 && load_factor < 1.0) ? load_factor : 0.5;
     CallScope s(db, default_scratch(c));
-    const GbSizing sz = group_by_i64_sizing(s.c, *key, nrows, expected_groups);
+    const GbSizing sz = group_by_i64_sizing(s.c, *key, nrows, expected_groups, nterms);
     s.c.scratch_reset();
     op_group_by_i64(s.c, *key, *value, nrows, prog, nterms, pred_cols, npred_cols, sz, lf, d_groups, capacity,
                     d_ngroups);

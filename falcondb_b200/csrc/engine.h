@@ -227,8 +227,8 @@ struct GbSizing {
 };
 // `expected_groups` when nonzero (no pass over the keys, no range), else the
 // sizing pass over the key column: estimate plus headroom, and the key range
-// (synchronises).
-GbSizing group_by_i64_sizing(Ctx& c, const fdb_dev_column& key, uint64_t n, uint64_t expected_groups);
+// (synchronises).  For an op_group_by_i64 with a WHERE of nterms terms.
+GbSizing group_by_i64_sizing(Ctx& c, const fdb_dev_column& key, uint64_t n, uint64_t expected_groups, int nterms);
 // Reserves its own scratch (on top of what is taken).
 void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& value, uint64_t n,
                      const fdb_pred_term* prog, int nterms, const fdb_dev_column* pred_cols,
@@ -265,9 +265,10 @@ struct KeyStats {
   uint64_t distinct = 0;
   bool has_range = false;  // false when every key is NULL (or there are none)
   int64_t kmin = 0, kmax = 0;
-  std::vector<uint32_t> parts;  // non-NULL keys per hash partition (below 2^32 keys)
+  std::vector<uint32_t> parts;  // non-NULL keys per hash partition; empty when not counted
 };
-KeyStats key_stats_i64(Ctx& c, const fdb_dev_column& key, uint64_t n);
+// `parts`: count the hash partitions if the keys look as if a GROUP BY would use them.
+KeyStats key_stats_i64(Ctx& c, const fdb_dev_column& key, uint64_t n, bool parts = false);
 
 // Zone maps (k_zone.cu, zone.cpp; pruning in zone_prune.cpp).
 // Fills d_out[0 .. zone_batches(nrows)) on stream s.

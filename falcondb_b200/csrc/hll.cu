@@ -3,8 +3,8 @@
 // Gandouet, Meunier, "HyperLogLog: the analysis of a near-optimal cardinality
 // estimation algorithm", 2007; 2^12 registers, standard error about 1.6 %),
 // and in the same pass the smallest and largest non-NULL key (NULL = a clear
-// validity bit, or INT64_MIN, which GROUP BY reads as NULL), and how many of them
-// fall into each hash partition (gb_partition).  One pass over the keys plus an
+// validity bit, or INT64_MIN, which GROUP BY reads as NULL), and, when asked, how many
+// of them fall into each hash partition (gb_partition).  One pass over the keys plus an
 // 18 KB device-to-host copy; synchronises the context stream.
 #include <cmath>
 #include <vector>
@@ -24,43 +24,69 @@ struct KeyStatsOut {
   unsigned int regs[kHllRegs];
   unsigned long long range[2];
   unsigned int parts[kGbParts];
+  unsigned int counted;  // parts[] are the keys' counts
 };
 
-__device__ __forceinline__ void hll_add(unsigned int* r, uint64_t h) {
+// Whether the key's register was empty.
+__device__ __forceinline__ bool hll_add(unsigned int* r, uint64_t h) {
   const uint32_t idx = (uint32_t)(h >> (64 - kHllBits));
   const uint64_t w = (h << kHllBits) | (1ull << (kHllBits - 1));  // bounds the run of zeros
-  atomicMax(&r[idx], (unsigned int)__clzll((long long)w) + 1u);
+  return atomicMax(&r[idx], (unsigned int)__clzll((long long)w) + 1u) == 0;
+}
+
+struct KeyColumn {
+  const int64_t* keys;
+  const uint64_t* validity;
+  uint64_t voff, n;
+  __device__ __forceinline__ bool valid(int64_t k, uint64_t row) const {
+    if (k == INT64_MIN) return false;
+    if (!validity) return true;
+    const uint64_t b = voff + row;
+    return (validity[b >> 6] >> (b & 63)) & 1ull;
+  }
+};
+
+// Whether the column's keys look worth counting per partition: one more shared
+// atomic per key (20M keys: 50 us, 43 without), used only by a GROUP BY of 32,768
+// groups or more (gb_partitions).  512 keys, the same for every CTA, in pairs
+// of neighbours spread over the column, decide:
+//   * too few values: the valid ones among the pairs' first keys fill less than 226
+//     registers in 256 (32,768 values fill 247 +- 3; 1300 values 226, Zipf keys fewer);
+//   * runs of equal keys, more than some 27 long (GbHashOp's CTA tables then take in
+//     most rows: 20M sorted ids of 50 rows each 0.88 ms, 0.95 by partitions).
+// All threads call, with r[] empty and block-wide ordered; r[] keeps the keys.
+constexpr int kLookThreads = 256;
+__device__ __forceinline__ bool parts_look_useful(const KeyColumn& c, const longlong2* pairs, uint64_t np,
+                                                  uint64_t head, unsigned int* r) {
+  const uint64_t p = (np / kLookThreads) * threadIdx.x + (threadIdx.x * 0x9E3779B1u >> 8) % (uint32_t)(np / kLookThreads);
+  const longlong2 k = pairs[p];
+  const bool vx = c.valid(k.x, head + 2 * p), vy = c.valid(k.y, head + 2 * p + 1);
+  const bool fresh = vx && hll_add(r, mix64((uint64_t)k.x ^ (1ull << 63)));
+  const int values = __syncthreads_count(fresh), valid = __syncthreads_count(vx);
+  const int runs = __syncthreads_count(vx && vy && k.x == k.y);
+  return values * 256 >= valid * 226 && runs * 256 <= valid * 246;
 }
 
 // Each thread takes 4 aligned pairs of keys per round (4 x 16-byte loads in
 // flight), so the pass runs near HBM speed; keys before the first 16-byte
 // boundary and after the last full pair are read one by one by thread 0 of
 // block 0 and the grid's tail.
-__global__ void __launch_bounds__(256) key_stats_kernel(const int64_t* __restrict__ keys, const uint64_t* validity,
-                                                        uint64_t voff, uint64_t n, KeyStatsOut* out) {
-  __shared__ unsigned int r[kHllRegs];
-  __shared__ unsigned int parts[kGbParts];
-  for (int i = threadIdx.x; i < kHllRegs; i += blockDim.x) r[i] = 0;
-  for (int i = threadIdx.x; i < (int)kGbParts; i += blockDim.x) parts[i] = 0;
-  __syncthreads();
+template <bool kParts>
+__device__ __forceinline__ void key_stats_rows(const KeyColumn& c, unsigned int* r, unsigned int* parts, uint64_t head,
+                                               KeyStatsOut* out) {
+  const int64_t* __restrict__ keys = c.keys;
+  const uint64_t n = c.n;
   uint64_t lo = ~0ull, hi = 0;
   auto take = [&](int64_t k, uint64_t row) {
     const uint64_t h = mix64((uint64_t)k ^ (1ull << 63));
     hll_add(r, h);
-    bool valid = k != INT64_MIN;
-    if (validity) {
-      const uint64_t b = voff + row;
-      valid = valid && ((validity[b >> 6] >> (b & 63)) & 1ull);
-    }
-    if (valid) {
+    if (c.valid(k, row)) {
       const uint64_t o = i64_ord_key(k);
       lo = o < lo ? o : lo;
       hi = o > hi ? o : hi;
-      atomicAdd(&parts[gb_partition(h)], 1u);
+      if (kParts) atomicAdd(&parts[gb_partition(h)], 1u);
     }
   };
-  // Head: rows before the first 16-byte aligned key.
-  const uint64_t head = umin64(n, (uint64_t)((16 - ((uintptr_t)keys & 15)) & 15) / 8);
   if (blockIdx.x == 0 && threadIdx.x == 0)
     for (uint64_t i = 0; i < head; ++i) take(keys[i], i);
   const longlong2* pairs = reinterpret_cast<const longlong2*>(keys + head);
@@ -91,9 +117,27 @@ __global__ void __launch_bounds__(256) key_stats_kernel(const int64_t* __restric
     if (lo != ~0ull) atomicMin(&out->range[0], (unsigned long long)lo);
     if (hi != 0) atomicMax(&out->range[1], (unsigned long long)hi);
   }
+}
+
+__global__ void __launch_bounds__(kLookThreads) key_stats_kernel(KeyColumn c, bool want_parts, KeyStatsOut* out) {
+  __shared__ unsigned int r[kHllRegs];
+  __shared__ unsigned int parts[kGbParts];
+  for (int i = threadIdx.x; i < kHllRegs; i += blockDim.x) r[i] = 0;
+  for (int i = threadIdx.x; i < (int)kGbParts; i += blockDim.x) parts[i] = 0;
+  __syncthreads();
+  // Head: rows before the first 16-byte aligned key.
+  const uint64_t head = umin64(c.n, (uint64_t)((16 - ((uintptr_t)c.keys & 15)) & 15) / 8);
+  const bool count =
+      want_parts && parts_look_useful(c, reinterpret_cast<const longlong2*>(c.keys + head), (c.n - head) / 2, head, r);
+  if (count)
+    key_stats_rows<true>(c, r, parts, head, out);
+  else
+    key_stats_rows<false>(c, r, parts, head, out);
   __syncthreads();
   for (int i = threadIdx.x; i < kHllRegs; i += blockDim.x)
     if (r[i]) atomicMax(&out->regs[i], r[i]);
+  if (!count) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) out->counted = 1;
   for (int i = threadIdx.x; i < (int)kGbParts; i += blockDim.x)
     if (parts[i]) atomicAdd(&out->parts[i], parts[i]);
 }
@@ -111,7 +155,7 @@ static uint64_t hll_estimate(const unsigned int* h, uint64_t n) {
   return std::min<uint64_t>(n, (uint64_t)std::ceil(e));
 }
 
-KeyStats key_stats_i64(Ctx& c, const fdb_dev_column& key, uint64_t n) {
+KeyStats key_stats_i64(Ctx& c, const fdb_dev_column& key, uint64_t n, bool parts) {
   KeyStats s;
   if (n == 0) {
     s.distinct = 1;
@@ -122,8 +166,8 @@ KeyStats key_stats_i64(Ctx& c, const fdb_dev_column& key, uint64_t n) {
   FDB_CUDA(cudaMemsetAsync(d, 0, sizeof(KeyStatsOut), c.stream));
   FDB_CUDA(cudaMemsetAsync(&d->range[0], 0xFF, 8, c.stream));
   const unsigned grid = (unsigned)umin64((n / 2 + 255) / 256 + 1, (uint64_t)c.sm_count * 8);
-  key_stats_kernel<<<grid, 256, 0, c.stream>>>(static_cast<const int64_t*>(key.values), key.validity,
-                                               key.validity_offset, n, d);
+  const KeyColumn col{static_cast<const int64_t*>(key.values), key.validity, key.validity_offset, n};
+  key_stats_kernel<<<grid, kLookThreads, 0, c.stream>>>(col, parts && n >= 4 * kLookThreads && n < (1ull << 32), d);
   FDB_CUDA(cudaGetLastError());
   KeyStatsOut h;
   HostReads reads(c);
@@ -135,7 +179,7 @@ KeyStats key_stats_i64(Ctx& c, const fdb_dev_column& key, uint64_t n) {
     s.kmin = (int64_t)(h.range[0] ^ (1ull << 63));
     s.kmax = (int64_t)(h.range[1] ^ (1ull << 63));
   }
-  if (n < (1ull << 32)) s.parts.assign(h.parts, h.parts + kGbParts);
+  if (h.counted) s.parts.assign(h.parts, h.parts + kGbParts);
   return s;
 }
 

@@ -1659,7 +1659,10 @@ static uint64_t gb_table_capacity(uint64_t expected_groups, double load_factor) 
   return cap;
 }
 
-GbSizing group_by_i64_sizing(Ctx& c, const fdb_dev_column& key, uint64_t n, uint64_t expected_groups) {
+// The rows and WHERE that the hash partitions take (gb_partitions).
+static bool gb_partition_rows(uint64_t n, int nterms) { return !nterms && n >= (1u << 20) && n < (1ull << 32); }
+
+GbSizing group_by_i64_sizing(Ctx& c, const fdb_dev_column& key, uint64_t n, uint64_t expected_groups, int nterms) {
   GbSizing s;
   if (expected_groups) {
     s.groups = expected_groups;
@@ -1687,7 +1690,7 @@ GbSizing group_by_i64_sizing(Ctx& c, const fdb_dev_column& key, uint64_t n, uint
       return s;
     }
   }
-  const KeyStats k = key_stats_i64(c, key, n);
+  const KeyStats k = key_stats_i64(c, key, n, gb_partition_rows(n, nterms));
   // 15 % headroom over the sketch (about nine standard errors).
   s.groups = std::min<uint64_t>(n, k.distinct * 115 / 100 + 64);
   s.has_range = k.has_range;
@@ -1726,8 +1729,9 @@ static size_t group_by_i64_scratch(const GbSizing& s, double load_factor) {
 // worth of them, and no partition with much more than its share of the rows (a
 // frequent key, whose partition one CTA would have to itself; GbHashOp's CTA
 // tables take such keys in).  Below a million rows the passes' fixed costs win.
+// The partitions are counted only where they look useful (parts_look_useful).
 static bool gb_partitions(const GbSizing& s, double load_factor, uint64_t n, int nterms) {
-  if (nterms || n < (1u << 20) || n >= (1ull << 32) || s.parts.size() != kGbParts) return false;
+  if (!gb_partition_rows(n, nterms) || s.parts.size() != kGbParts) return false;
   if (s.groups < 64ull * kGbParts || s.groups > 2ull * kGbParts * (kPartSlots * 5 / 8)) return false;
   if (gb_dense_slots(s, gb_load_factor(load_factor))) return false;
   uint64_t total = 0, most = 0;

@@ -1080,7 +1080,7 @@ static void run_aggregates(Plan& plan, const Rel& rel, const Query& q, fdb_resul
       fdb_group_i64* d = plan.dev<fdb_group_i64>(cap);
       uint64_t* dn = plan.dev<uint64_t>(1);
       plan.c.scratch_reset();
-      const GbSizing sz = group_by_i64_sizing(plan.c, col.dev, rel.nrows, 0);
+      const GbSizing sz = group_by_i64_sizing(plan.c, col.dev, rel.nrows, 0, (int)prog.size());
       plan.c.scratch_reset();
       op_group_by_i64(plan.c, col.dev, col.dev, rel.nrows, prog.data(), (int)prog.size(), pcols.data(),
                       (int)pcols.size(), sz, 0.5, d, cap, dn);
@@ -1226,7 +1226,7 @@ static void run_group_by(Plan& plan, const Rel& rel, const Query& q, fdb_result*
     uint64_t* dn = plan.dev<uint64_t>(1);
     std::vector<fdb_group_i64> groups;
     if (rel.nrows > 0) {
-      const GbSizing sz = group_by_i64_sizing(plan.c, key.dev, rel.nrows, 0);
+      const GbSizing sz = group_by_i64_sizing(plan.c, key.dev, rel.nrows, 0, (int)prog.size());
       op_group_by_i64(plan.c, key.dev, rel.cols[vc].dev, rel.nrows, prog.data(), (int)prog.size(), pcols.data(),
                       (int)pcols.size(), sz, 0.5, d, cap, dn);
       groups = plan.to_host(d, plan.checked_one(dn));
