@@ -803,25 +803,31 @@ constexpr uint32_t kDenseProbe = FDB_GBD_PROBE;
 constexpr uint32_t kDenseSumCopies = FDB_GBD_SUMSPLIT;
 static_assert((kDenseSumCopies & (kDenseSumCopies - 1)) == 0, "SUM copies: a power of two");
 // Launch shape of the two-column instance (key, value): tile rows, stages,
-// consumer warps.  Two CTAs of sixteen warps per SM, one row per thread and tile.
+// consumer warps.  Two CTAs of sixteen warps per SM, two rows per thread and tile.
 // What spills goes to the global table in four REDs, so a larger CTA table pays
 // (2048 slots instead of 1024: 40 instead of 45 % of 10M Zipf(1.1) keys' rows
 // spill) as long as a frequent key's rows are merged (warp_slot_rows) and 32 warps
 // stay resident.  Against three CTAs of 1024 slots and eight warps with four rows
-// per thread, GROUP BY in all: 100M rows of 10M Zipf keys 1.72 -> 1.54 ms, 20M of
-// 5000 Zipf keys 0.375 -> 0.305, 60M of 800 uniform keys 0.480 -> 0.445.  Two stages
-// instead of three: 1.60, 0.319, 0.500; 4096 slots in one CTA of 24 warps: 1.93,
-// 0.334, 0.478; 20 warps (registers leave one CTA): 2.08, 0.390, 0.636; merging at
-// the old shape: 1.94, 0.319, 0.511.
+// per thread, GROUP BY in all: 20M rows of 5000 Zipf keys 0.478 -> 0.388 ms, 60M of
+// 800 uniform keys 0.642 -> 0.543, of 200 uniform keys 0.584 -> 0.601.  Tiles of 512
+// rows, so one row per thread between two waits: 60M rows of 800 keys 0.581, of 200
+// 0.619, of 5000 Zipf keys 0.952.  Losing shapes, of 100M rows of 10M Zipf keys (1.54
+// ms), 20M of 5000 Zipf (0.305) and 60M of 800 uniform (0.445), kernels alone: 4096
+// slots in one CTA of 24 warps 1.93, 0.334, 0.478; 20 warps (registers leave one CTA)
+// 2.08, 0.390, 0.636; merging at the old shape 1.94, 0.319, 0.511.
 #ifndef FDB_GBD_TR
-#define FDB_GBD_TR 512
+#define FDB_GBD_TR 1024
 #endif
 #ifndef FDB_GBD_ST
-#define FDB_GBD_ST 3
+#define FDB_GBD_ST 2
 #endif
 #ifndef FDB_GBD_NCW
 #define FDB_GBD_NCW 16
 #endif
+// Fewer rows than this leave CTAs without tiles: half as large ones (this kernel, 3000
+// keys: 100,000 rows 18.7 us, 27.5 with whole ones; 600,000 27.3 and 31.6; 1M 40.3 and
+// 35.3).
+constexpr uint64_t kDenseSmallRows = 700'000;
 // Tiles from one look at whether a warp's rows are worth merging to the next.
 constexpr uint32_t kDenseMergeTiles = 16;
 
@@ -985,9 +991,13 @@ struct GbDenseOp {
             atomicExch(p.err, kErrCapacity);
           } else {
             k = (uint32_t)kk;
-            const uint32_t h = smem_dense_home(k);
-            j = smem_dense_slot_from(tab, k, h, tab.k1[h]);
-            spill = j < 0;
+            if (p.slots <= kDenseSmemSlots) {  // every key has its own slot: nothing to probe
+              j = (int)k;
+            } else {
+              const uint32_t h = smem_dense_home(k);
+              j = smem_dense_slot_from(tab, k, h, tab.k1[h]);
+              spill = j < 0;
+            }
           }
         }
       }
@@ -1005,7 +1015,7 @@ struct GbDenseOp {
     const SDTab tab = sdtab(sm);
     consumer_bar(nct);
     for (uint32_t j = ctid; j < kDenseSmemSlots; j += nct) {
-      const unsigned int k1 = tab.k1[j];
+      const unsigned int k1 = p.slots <= kDenseSmemSlots ? (tab.count[j] ? j + 1 : 0u) : tab.k1[j];
       if (k1) dslot_merge(p.table + (k1 - 1), tab, j);
     }
     if (ctid == 0 && tab.count[kDenseSmemSlots]) dslot_merge(p.null_slot, tab, kDenseSmemSlots);
@@ -1790,7 +1800,12 @@ void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& va
     p.err = c.d_err;
     if (n > 0) {
       switch (nc) {
-        case 2: launch_stream_gb<GbDenseOp, 2, FDB_GBD_TR, FDB_GBD_ST, FDB_GBD_NCW>(c, all, n, p, GbDenseOp::kSmem); break;
+        case 2:
+          if (n < kDenseSmallRows)
+            launch_stream_gb<GbDenseOp, 2, FDB_GBD_TR / 2, FDB_GBD_ST + 1, FDB_GBD_NCW>(c, all, n, p, GbDenseOp::kSmem);
+          else
+            launch_stream_gb<GbDenseOp, 2, FDB_GBD_TR, FDB_GBD_ST, FDB_GBD_NCW>(c, all, n, p, GbDenseOp::kSmem);
+          break;
         // Still two CTAs per SM beside the WHERE columns (40M rows, one column:
         // 800 uniform keys 0.56 ms, 0.74 with tiles of 1024 and one CTA).
         case 3: launch_stream_gb<GbDenseOp, 3, 512, 2, 16>(c, all, n, p, GbDenseOp::kSmem); break;
