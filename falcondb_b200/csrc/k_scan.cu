@@ -111,12 +111,14 @@ struct TileShape {
   static constexpr int NCW = 8;
 };
 struct ScanAggParams {
-  PredProg prog;
+  union {
+    PredProg prog;
+    WhereProg where;      // FilterAggOp: the same program, decoded
+  };
   ScanCols sc;
   int32_t naggs;
   int32_t func[4];
   int32_t acol[4];
-  WhereProg where;        // FilterAggOp: the same program, decoded
   uint32_t f_agg_f64;     // bit a: aggregate a's column is FLOAT64
   AggAcc* partials;       // [gridDim.x * 4]
   unsigned int* ticket;   // zero on entry; reset by the last CTA
@@ -319,19 +321,23 @@ __device__ __forceinline__ void fold_value(AggAcc& a, int f, T v) {
 //   * an INT64 SUM / AVG keeps the sum of the values' low 32-bit halves
 //     (unsigned) in slo and of their high halves (signed) in shi, so that
 //     the value is shi * 2^32 + slo; exact while a thread folds fewer than
-//     2^32 rows (the host only takes this path below 2^40 rows);
+//     2^32 rows;
 //   * a FLOAT64 MIN / MAX keeps the running value in f (+inf / -inf before the
 //     first row) and compares doubles: NaN compares false and never takes
 //     part (f64::min / max), and on equal values the sign bits are combined
 //     so that +0.0 wins a MAX and -0.0 a MIN, as their order keys do.
+// The program comes in three forms, each an instance: none; one comparison
+// (where_one); any (where_mask, and NULLs).  In one instance for all, the first two
+// paid for the third's loop, its parameter reads by index and its code size: INT64
+// SUM under one comparison over 50M rows 104 us, now 77; two INT64 columns without a
+// WHERE 184, now 145; SUM, AVG, MAX under one comparison 179, now 150.
+//
 // FilterAggOp's launch shape: 2048-row tiles (1024 with three or four columns,
-// so that three CTAs' rings still fit an SM), two stages, and registers held to
-// three resident CTAs per SM (72, no spills).  Bound by instruction issue and
+// so that three CTAs' rings still fit an SM), two or three stages, and registers
+// held to three resident CTAs per SM (no spills).  Bound by instruction issue and
 // by latency at 24 consumer warps per SM, not by HBM.  COUNT, SUM(score),
-// AVG(salary), MAX(score): WHERE score > 50 over 100M rows 0.318 ms (0.362 with
-// a one-compare form that tested four outcomes per row and selected around
-// every MAX); WHERE score > 50 AND salary < 150000 over 33.3M rows with NULL
-// scores 0.176 ms, where ScanAggOp takes 0.791 ms.
+// AVG(salary), MAX(score): WHERE score > 50 AND salary < 150000 over 33.3M rows with
+// NULL scores 0.176 ms, where ScanAggOp takes 0.791 ms.
 #ifndef FDB_FA_TR
 #define FDB_FA_TR 2048
 #endif
@@ -341,6 +347,7 @@ __device__ __forceinline__ void fold_value(AggAcc& a, int f, T v) {
 #ifndef FDB_FA_MINB
 #define FDB_FA_MINB 3
 #endif
+template <WhereForm kForm>
 struct FilterAggOp : ScanAggOp {
   static constexpr int R = 4;
 
@@ -360,7 +367,7 @@ struct FilterAggOp : ScanAggOp {
   }
 
   static __device__ __forceinline__ void prefetch(const Params& p, uint64_t row0, uint32_t rows) {
-    prefetch_valid(p.where.nullable, p.sc.cols, row0, rows);
+    if constexpr (kForm == kWhereAny) prefetch_valid(p.where.nullable, p.sc.cols, row0, rows);
   }
 
   template <bool kFull, typename T, class Acc>
@@ -438,8 +445,13 @@ struct FilterAggOp : ScanAggOp {
       i[j] = b + (uint32_t)j * kStride + (uint32_t)ctid;
       ok |= (kFull || i[j] < rows ? 1u : 0u) << j;
     }
-    const uint32_t valid = valid_masks<kFull, R, kStride>(p.where.nullable, p.sc.cols, acc, i, ok);
-    const uint32_t pass = where_mask<kFull, R>(p.where, acc, p.sc.cols, i, ok, valid);
+    uint32_t valid = 0, pass = ok;
+    if constexpr (kForm == kWhereOne) {
+      pass = where_one<kFull, R>(p.where, acc, i, ok);
+    } else if constexpr (kForm == kWhereAny) {
+      valid = valid_masks<kFull, R, kStride>(p.where.nullable, p.sc.cols, acc, i, ok);
+      pass = where_mask<kFull, R>(p.where, acc, p.sc.cols, i, ok, valid);
+    }
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
       if (a >= p.naggs) break;
@@ -448,7 +460,7 @@ struct FilterAggOp : ScanAggOp {
         st.a[a].n += (uint64_t)__popc(pass);
         continue;
       }
-      const uint32_t m = pass & (valid >> (p.acol[a] * R));
+      const uint32_t m = kForm != kWhereAny ? pass : pass & (valid >> (p.acol[a] * R));
       if (f == FDB_AGG_COUNT)
         st.a[a].n += (uint64_t)__popc(m);
       else if ((p.f_agg_f64 >> a) & 1u)
@@ -707,20 +719,35 @@ static void launch_stream_nc(Ctx& c, const fdb_dev_column* cols, int ncols, uint
   }
 }
 
-// FilterAggOp over p's program and aggregates.  Its split INT64 sums are exact
-// below 2^32 rows per thread, so from 2^40 rows on the interpreter takes over.
-static void launch_filter_agg(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n, ScanAggParams& p) {
-  if (n >= (1ull << 40)) {
-    launch_stream_nc<ScanAggOp>(c, cols, ncols, n, p, ScanAggOp::kSmem);
-    return;
-  }
-  fill_where(p.where, p.prog, p.sc.cols, ncols);
+// FilterAggOp over the program and p's aggregates.  Stages and resident CTAs: one
+// column's tiles need a third stage (one INT64 comparison over 50M rows 77 us, 80
+// with two); three and four columns without a program, or with one comparison,
+// take three where they pay (50M rows, us, three stages / two: three SUMs 184 / 186;
+// four MIN / MAX 255 / 254, 12M 78 / 83; four SUMs 254 / 257, 3M 36 / 40; 2048-row
+// tiles: 306, 98, 248, 34).
+template <WhereForm kForm>
+static void launch_filter_agg_nc(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n, const ScanAggParams& p) {
+  using Op = FilterAggOp<kForm>;
   constexpr int kTr = FDB_FA_TR, kSt = FDB_FA_STAGES, kMin = FDB_FA_MINB;
+  constexpr bool kAny = kForm == kWhereAny;
   switch (ncols) {
-    case 1: launch_stream<FilterAggOp, 1, kTr, 8, kSt, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
-    case 2: launch_stream<FilterAggOp, 2, kTr, 8, kSt, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
-    case 3: launch_stream<FilterAggOp, 3, kTr / 2, 8, kSt, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
-    default: launch_stream<FilterAggOp, 4, kTr / 2, 8, kSt, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
+    case 1: launch_stream<Op, 1, kTr, 8, kSt + 1, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
+    case 2: launch_stream<Op, 2, kTr, 8, kSt, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
+    case 3: launch_stream<Op, 3, kTr / 2, 8, kAny ? kSt : kSt + 1, kMin>(c, cols, n, p, ScanAggOp::kSmem); break;
+    default:
+      launch_stream<Op, 4, kTr / 2, 8, kForm == kWhereNone ? kSt + 1 : kSt, kAny ? kMin : 2>(c, cols, n, p,
+                                                                                           ScanAggOp::kSmem);
+  }
+}
+
+// Its split INT64 sums are exact below 2^32 rows per thread: no device holds 2^40 rows.
+static void launch_filter_agg(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n, const PredProg& prog,
+                              ScanAggParams& p) {
+  fill_where(p.where, prog, p.sc.cols, ncols);
+  switch (where_form(p.where)) {
+    case kWhereNone: launch_filter_agg_nc<kWhereNone>(c, cols, ncols, n, p); break;
+    case kWhereOne: launch_filter_agg_nc<kWhereOne>(c, cols, ncols, n, p); break;
+    default: launch_filter_agg_nc<kWhereAny>(c, cols, ncols, n, p); break;
   }
 }
 
@@ -771,7 +798,8 @@ void op_aggregate(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,
   ScanAggParams p;
   std::memset(&p, 0, sizeof(p));
   fill_cols(p.sc, cols, ncols, n);
-  fill_prog(p.prog, prog, nterms, ncols);
+  PredProg pp;
+  fill_prog(pp, prog, nterms, ncols);
   p.naggs = naggs;
   for (int a = 0; a < naggs; ++a) {
     const int f = aggs[a].func;
@@ -802,7 +830,7 @@ void op_aggregate(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,
   }
   for (int a = 0; a < naggs; ++a)
     if (aggs[a].func != FDB_AGG_COUNT_STAR && cols[aggs[a].col].dtype == FDB_FLOAT64) p.f_agg_f64 |= 1u << a;
-  launch_filter_agg(c, cols, ncols, n, p);
+  launch_filter_agg(c, cols, ncols, n, pp, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -899,7 +927,8 @@ void op_filter_count(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,
   ScanAggParams p;
   std::memset(&p, 0, sizeof(p));
   fill_cols(p.sc, cols, ncols, n);
-  fill_prog(p.prog, prog, nterms, ncols);
+  PredProg pp;
+  fill_prog(pp, prog, nterms, ncols);
   p.naggs = 1;
   p.func[0] = FDB_AGG_COUNT_STAR;
   p.acol[0] = 0;
@@ -910,6 +939,7 @@ void op_filter_count(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,
   // `col op literal` over one NULL-free numeric column.
   if (ncols == 1 && nterms == 1 && prog[0].kind == FDB_TERM_CMP && prog[0].col == 0 &&
       cols[0].validity == nullptr && cols[0].dtype != FDB_UTF8) {
+    p.prog = pp;
     if (cols[0].dtype == FDB_FLOAT64)
       launch_cmp_count<double, double>(c, cols, n, p, prog[0].op);
     else if (prog[0].lit_type == FDB_FLOAT64)
@@ -918,7 +948,7 @@ void op_filter_count(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,
       launch_cmp_count<int64_t, int64_t>(c, cols, n, p, prog[0].op);
     return;
   }
-  launch_filter_agg(c, cols, ncols, n, p);
+  launch_filter_agg(c, cols, ncols, n, pp, p);
 }
 
 void op_distinct_codes(Ctx& c, const fdb_dev_column* cols, int ncols, uint64_t n,

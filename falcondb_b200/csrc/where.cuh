@@ -41,8 +41,30 @@ struct WhereTerm {
 struct WhereProg {
   int32_t n;
   uint32_t nullable;   // bit c: column c has validity words
+  // One comparison of an INT64 column with an int64 (where_one): the values
+  // [one_lo, one_lo + one_span], or with one_not (all ones) those outside.
+  uint32_t one_not;
+  int64_t one_lo;
+  uint64_t one_span;
   WhereTerm t[FDB_MAX_TERMS];
 };
+
+// x op lit over int64, as such a range.
+inline void fill_where_range(WhereProg& w, int op, int64_t lit) {
+  int64_t lo = INT64_MIN, hi = INT64_MAX;
+  bool outside = false;
+  switch (op) {
+    case FDB_EQ: lo = hi = lit; break;
+    case FDB_NE: lo = hi = lit; outside = true; break;
+    case FDB_LE: hi = lit; break;
+    case FDB_GT: hi = lit; outside = true; break;
+    case FDB_GE: lo = lit; break;
+    default: lo = lit; outside = true;  // <
+  }
+  w.one_lo = lo;
+  w.one_span = (uint64_t)hi - (uint64_t)lo;
+  w.one_not = outside ? 0xFFFFFFFFu : 0u;
+}
 
 // A checked program (fill_prog) over columns `cols`, decoded.
 inline void fill_where(WhereProg& w, const PredProg& prog, const DevCol* cols, int ncols) {
@@ -81,6 +103,16 @@ inline void fill_where(WhereProg& w, const PredProg& prog, const DevCol* cols, i
         }
     }
   }
+  if (w.n == 1 && w.t[0].kind == kWhereI64) fill_where_range(w, w.t[0].op, w.t[0].lit_i);
+}
+
+// Programs that scans of NULL-free columns decide with less than where_mask: none,
+// and one comparison of a numeric column (where_one).
+enum WhereForm { kWhereNone, kWhereOne, kWhereAny };
+inline WhereForm where_form(const WhereProg& w) {
+  if (w.nullable || w.n > 1) return kWhereAny;
+  if (w.n == 0) return kWhereNone;
+  return w.t[0].kind <= kWhereI64AsF64 ? kWhereOne : kWhereAny;
 }
 
 // x[j] op lit for R values, the operator decided once (floating compares are
@@ -231,6 +263,35 @@ __device__ __forceinline__ uint32_t where_mask(const WhereProg& w, const Acc& ac
     }
   }
   return kFull ? top : (top & ok);
+}
+
+// where_mask for one comparison (kWhereOne), which is the program's first term: its
+// fields are read at fixed places of the parameters.
+template <bool kFull, int R, class Acc>
+__device__ __forceinline__ uint32_t where_one(const WhereProg& w, const Acc& acc, const uint32_t (&i)[R],
+                                              uint32_t ok) {
+  const WhereTerm& t = w.t[0];
+  uint32_t m = 0;
+  if (t.kind == kWhereF64) {
+    double x[R];
+    where_load<kFull, R>(x, acc, t.col, i, ok);
+    m = cmp_mask<R, double>(t.op, x, t.lit_f);
+  } else {
+    int64_t y[R];
+    where_load<kFull, R>(y, acc, t.col, i, ok);
+    if (t.kind == kWhereI64) {
+      const uint64_t lo = (uint64_t)w.one_lo, span = w.one_span;
+#pragma unroll
+      for (int j = 0; j < R; ++j) m |= ((uint64_t)y[j] - lo <= span ? 1u : 0u) << j;
+      m = (m ^ w.one_not) & ((1u << R) - 1u);
+    } else {
+      double x[R];
+#pragma unroll
+      for (int j = 0; j < R; ++j) x[j] = (double)y[j];
+      m = cmp_mask<R, double>(t.op, x, t.lit_f);
+    }
+  }
+  return kFull ? m : (m & ok);
 }
 
 }  // namespace fdb
