@@ -1146,7 +1146,9 @@ __global__ void __launch_bounds__(kCompactThreads)
   uint64_t total;
   const uint32_t base = (uint32_t)block_exclusive_scan<uint64_t>(cnt, sm, &total);
   const uint64_t off = offsets[blockIdx.x];
-  if (total <= kSparseRows) {
+  // The last chunk may have few rows, most of which pass: its words are walked too.
+  const uint64_t words_here = nwords - c0 < kChunkWords ? nwords - c0 : kChunkWords;
+  if (total <= kSparseRows && total <= words_here * 32) {
     uint32_t o = base;
 #pragma unroll
     for (int j = 0; j < kWordsPerThread; ++j)
