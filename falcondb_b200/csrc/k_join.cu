@@ -489,8 +489,12 @@ HashTable* op_join_build(Ctx& c, const fdb_dev_column& key, const fdb_dev_column
   h->span = span;
   const JoinMode mode = join_mode(*h);
   if (n > 0) {
-    const unsigned blocks =
-        (unsigned)umin64((n + 256 * kInsertRows - 1) / (256 * kInsertRows), (uint64_t)c.sm_count * 16);
+    // Four rows per thread once there are four CTAs per SM (1000 rows: the insert 3.8 us
+    // in four CTAs, 8.0 in one; 1M rows of 500,000 keys, the build 154 us, 165 with
+    // one row per thread).
+    const uint64_t whole = (n + 256 * kInsertRows - 1) / (256 * kInsertRows);
+    const uint64_t spread = umin64((n + 255) / 256, (uint64_t)c.sm_count * 4);
+    const unsigned blocks = (unsigned)umin64(whole > spread ? whole : spread, (uint64_t)c.sm_count * 16);
     join_insert_kernel<<<blocks, 256, 0, c.stream>>>(
         static_cast<const int64_t*>(key.values), key.validity, key.validity_offset,
         static_cast<const int64_t*>(payload.values), payload.validity, payload.validity_offset, n,
