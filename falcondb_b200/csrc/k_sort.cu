@@ -644,7 +644,8 @@ static void radix_sort_pairs(Ctx& c, uint32_t m, KeysFn keys_fn, uint32_t* rows_
     else  // the digits the last scatter wrote
       radix_hist_digits_kernel<<<(ntiles + kDigitHistWarps - 1) / kDigitHistWarps, kDigitHistWarps * 32, 0,
                                  c.stream>>>(dg, m, ntiles, hist);
-    sort_scan_sums_kernel<<<(unsigned)nb, kScanT, 0, c.stream>>>(hist, hn, bsum);
+    // One block (up to 65,536 keys) adds no sums.
+    if (nb > 1) sort_scan_sums_kernel<<<(unsigned)nb, kScanT, 0, c.stream>>>(hist, hn, bsum);
     sort_scan_apply_kernel<<<(unsigned)nb, kScanT, 0, c.stream>>>(hist, hn, bsum);
     const bool last = p + 1 == npass;
     const bool direct = rows_out && last;  // rows go straight to the output; keys are not needed
@@ -778,11 +779,10 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
   const uint64_t n1 = (uint64_t)p.parts1 * p.cap1, leaves = (uint64_t)p.parts1 * std::max(1u, p.parts2);
   MsdMap* map1 = static_cast<MsdMap*>(c.scratch_take(sizeof(MsdMap)));
   // State words, what varies (for the radix passes), and the counters of both
-  // levels, cleared together.
+  // levels, a multiple of four words, which the sample kernel clears.
   const uint32_t counters = 64 + p.parts1 + (p.parts2 ? (uint32_t)leaves : 0u);
   uint32_t* state = static_cast<uint32_t*>(c.scratch_take(counters * 4));
   uint32_t *cur1 = state + 64, *cur2 = cur1 + p.parts1;
-  FDB_CUDA(cudaMemsetAsync(state, 0, counters * 4, c.stream));
   // Two radix passes beat the sample sort at any size, three up to a few million
   // pairs (1.9M int64 keys of 18 bits: 179 us against 204; 20M: 760 against 600).
   const int few_bytes = m < 4'000'000 ? 3 : 2;
@@ -790,10 +790,10 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
   auto log2 = [](uint32_t x) { return 31 - __builtin_clz(x); };
   if (p.samples > 1024 * kMsdSampleItems)
     msd_sample_kernel<Src, 2 * kMsdSampleItems><<<1, 1024, sizeof(MsdSampleSmem), c.stream>>>(
-        src, m, log2(p.samples), p.parts1, run, few_bytes, map1, state);
+        src, m, log2(p.samples), p.parts1, run, few_bytes, map1, state, counters);
   else
     msd_sample_kernel<Src, kMsdSampleItems><<<1, 1024, sizeof(MsdSampleSmem), c.stream>>>(
-        src, m, log2(p.samples), p.parts1, run, few_bytes, map1, state);
+        src, m, log2(p.samples), p.parts1, run, few_bytes, map1, state, counters);
   // The radix passes' key kernel runs only when the sample showed repeats; one
   // copy then tells the host which way to go.
   const size_t mark = c.scratch_top;
