@@ -944,6 +944,9 @@ __device__ __forceinline__ int smem_dense_slot_from(const SDTab& t, uint32_t k, 
   return -1;
 }
 
+// kDirect: at most kDenseSmemSlots key values, each with its own CTA slot, nothing to
+// probe (an instance of its own: the test per row cost 100M rows of 5000 Zipf keys 2 %).
+template <bool kDirect>
 struct GbDenseOp {
   using Params = GbDenseParams;
   struct Local {
@@ -991,7 +994,7 @@ struct GbDenseOp {
             atomicExch(p.err, kErrCapacity);
           } else {
             k = (uint32_t)kk;
-            if (p.slots <= kDenseSmemSlots) {  // every key has its own slot: nothing to probe
+            if constexpr (kDirect) {
               j = (int)k;
             } else {
               const uint32_t h = smem_dense_home(k);
@@ -1015,7 +1018,7 @@ struct GbDenseOp {
     const SDTab tab = sdtab(sm);
     consumer_bar(nct);
     for (uint32_t j = ctid; j < kDenseSmemSlots; j += nct) {
-      const unsigned int k1 = p.slots <= kDenseSmemSlots ? (tab.count[j] ? j + 1 : 0u) : tab.k1[j];
+      const unsigned int k1 = kDirect ? (tab.count[j] ? j + 1 : 0u) : tab.k1[j];
       if (k1) dslot_merge(p.table + (k1 - 1), tab, j);
     }
     if (ctid == 0 && tab.count[kDenseSmemSlots]) dslot_merge(p.null_slot, tab, kDenseSmemSlots);
@@ -1496,10 +1499,30 @@ static void launch_stream_gb(Ctx& c, const fdb_dev_column* cols, uint64_t n,
   const uint64_t want =
       ntiles ? (ntiles + kGbTilesPerCta - 1) / kGbTilesPerCta : (n + NCW * 32 * 8 - 1) / (NCW * 32 * 8);
   constexpr int kKind =
-      std::is_same<Op, GbDenseOp>::value || std::is_same<Op, GbHashOp>::value ? FDB_TUNE_GROUP_I64 : FDB_TUNE_GROUP;
+      std::is_same<Op, GbDenseOp<false>>::value || std::is_same<Op, GbDenseOp<true>>::value ||
+              std::is_same<Op, GbHashOp>::value
+          ? FDB_TUNE_GROUP_I64
+          : FDB_TUNE_GROUP;
   const int grid = tuned_grid(c.tune.op[kKind], c.sm_count, per_sm, 4, want, n);
   kern<<<grid, (NCW + 1) * 32, smem, c.stream>>>(src, p, c.d_err, op_off);
   FDB_CUDA(cudaGetLastError());
+}
+
+template <bool kDirect>
+static void launch_dense(Ctx& c, const fdb_dev_column* cols, int nc, uint64_t n, const GbDenseParams& p) {
+  using Op = GbDenseOp<kDirect>;
+  switch (nc) {
+    case 2:
+      if (n < kDenseSmallRows)
+        launch_stream_gb<Op, 2, FDB_GBD_TR / 2, FDB_GBD_ST + 1, FDB_GBD_NCW>(c, cols, n, p, Op::kSmem);
+      else
+        launch_stream_gb<Op, 2, FDB_GBD_TR, FDB_GBD_ST, FDB_GBD_NCW>(c, cols, n, p, Op::kSmem);
+      break;
+    // Still two CTAs per SM beside the WHERE columns (40M rows, one column:
+    // 800 uniform keys 0.56 ms, 0.74 with tiles of 1024 and one CTA).
+    case 3: launch_stream_gb<Op, 3, 512, 2, 16>(c, cols, n, p, Op::kSmem); break;
+    default: launch_stream_gb<Op, 4, 384, 2, 12>(c, cols, n, p, Op::kSmem); break;
+  }
 }
 
 static void gb_fill_prog(PredProg& pp, const fdb_pred_term* prog, int nterms, int ncols, int col_shift) {
@@ -1799,18 +1822,10 @@ void op_group_by_i64(Ctx& c, const fdb_dev_column& key, const fdb_dev_column& va
     p.null_slot = table + slots;
     p.err = c.d_err;
     if (n > 0) {
-      switch (nc) {
-        case 2:
-          if (n < kDenseSmallRows)
-            launch_stream_gb<GbDenseOp, 2, FDB_GBD_TR / 2, FDB_GBD_ST + 1, FDB_GBD_NCW>(c, all, n, p, GbDenseOp::kSmem);
-          else
-            launch_stream_gb<GbDenseOp, 2, FDB_GBD_TR, FDB_GBD_ST, FDB_GBD_NCW>(c, all, n, p, GbDenseOp::kSmem);
-          break;
-        // Still two CTAs per SM beside the WHERE columns (40M rows, one column:
-        // 800 uniform keys 0.56 ms, 0.74 with tiles of 1024 and one CTA).
-        case 3: launch_stream_gb<GbDenseOp, 3, 512, 2, 16>(c, all, n, p, GbDenseOp::kSmem); break;
-        default: launch_stream_gb<GbDenseOp, 4, 384, 2, 12>(c, all, n, p, GbDenseOp::kSmem); break;
-      }
+      if (slots <= kDenseSmemSlots)
+        launch_dense<true>(c, all, nc, n, p);
+      else
+        launch_dense<false>(c, all, nc, n, p);
     }
     dense_chunk_count_kernel<<<(unsigned)nchunks, kDenseCompactThreads, 0, c.stream>>>(table, slots, chunk_off);
     FDB_CUDA(cudaGetLastError());
