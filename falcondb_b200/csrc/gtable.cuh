@@ -142,7 +142,9 @@ __device__ __forceinline__ fdb_group_i64 gslot_group(uint64_t skey, const GSlot&
 
 // The lanes of a warp whose rows go to the same CTA slot (j; -1: none), merged
 // before the shared-memory atomics: the first of them gets their number and the
-// sum of their values, the others 0 rows.  All 32 lanes call.
+// sum of their values, the others 0 rows.  All 32 lanes call.  The method is the
+// known one for reducing by key within a warp: a match gives each lane its peers, and
+// in each round a lane adds its next live peer's value and every other peer drops out.
 struct SlotRows {
   uint32_t rows;
   double sum;

@@ -795,13 +795,6 @@ constexpr uint64_t kDenseMaxSlots = 1ull << 31;  // slot indices (and index + 1)
 #define FDB_GBD_PROBE 4
 #endif
 constexpr uint32_t kDenseProbe = FDB_GBD_PROBE;
-// Copies of each CTA slot's SUM, picked by lane: lanes of one warp that add to
-// the same hot slot then contend on up to kDenseSumCopies addresses, not one.
-#ifndef FDB_GBD_SUMSPLIT
-#define FDB_GBD_SUMSPLIT 1
-#endif
-constexpr uint32_t kDenseSumCopies = FDB_GBD_SUMSPLIT;
-static_assert((kDenseSumCopies & (kDenseSumCopies - 1)) == 0, "SUM copies: a power of two");
 // Launch shape of the two-column instance (key, value): tile rows, stages,
 // consumer warps.  Two CTAs of sixteen warps per SM, two rows per thread and tile.
 // What spills goes to the global table in four REDs, so a larger CTA table pays
@@ -815,15 +808,7 @@ static_assert((kDenseSumCopies & (kDenseSumCopies - 1)) == 0, "SUM copies: a pow
 // ms), 20M of 5000 Zipf (0.305) and 60M of 800 uniform (0.445), kernels alone: 4096
 // slots in one CTA of 24 warps 1.93, 0.334, 0.478; 20 warps (registers leave one CTA)
 // 2.08, 0.390, 0.636; merging at the old shape 1.94, 0.319, 0.511.
-#ifndef FDB_GBD_TR
-#define FDB_GBD_TR 1024
-#endif
-#ifndef FDB_GBD_ST
-#define FDB_GBD_ST 2
-#endif
-#ifndef FDB_GBD_NCW
-#define FDB_GBD_NCW 16
-#endif
+constexpr int kDenseTile = 1024, kDenseStages = 2, kDenseWarps = 16;
 // Fewer rows than this leave CTAs without tiles: half as large ones (this kernel, 3000
 // keys: 100,000 rows 18.7 us, 27.5 with whole ones; 600,000 27.3 and 31.6; 1M 40.3 and
 // 35.3).
@@ -841,27 +826,19 @@ struct GbDenseParams {
   int* err;
 };
 
-// MIN / MAX checked first against one 8-byte word holding the high halves of
-// both order keys (1), or against the two 64-bit keys (0).
-#ifndef FDB_GBD_MMHI
-#define FDB_GBD_MMHI 1
-#endif
-
-// Shared-memory bytes of the CTA table: kDenseSumCopies SUM arrays, then
-// nmin, max, the packed high halves, k1, count (slot kDenseSmemSlots is the
-// NULL group).
-constexpr size_t kDenseSmemBytes = (size_t)(kDenseSmemSlots + 1) * (8 * kDenseSumCopies + 32);
+// Shared-memory bytes of the CTA table: sum, nmin, max, the packed high halves, k1,
+// count (slot kDenseSmemSlots is the NULL group).
+constexpr size_t kDenseSmemBytes = (size_t)(kDenseSmemSlots + 1) * 40;
 
 __device__ __forceinline__ SDTab sdtab(unsigned char* sm) {
   constexpr uint32_t S = kDenseSmemSlots + 1;
-  constexpr size_t kSums = (size_t)8 * S * kDenseSumCopies;
   SDTab t;
-  t.sum = reinterpret_cast<double*>(sm);  // copy c of slot j: sum[c * S + j]
-  t.nmin = reinterpret_cast<unsigned long long*>(sm + kSums);
-  t.max = reinterpret_cast<unsigned long long*>(sm + kSums + 8 * S);
-  t.mmhi = reinterpret_cast<unsigned int*>(sm + kSums + 16 * S);
-  t.k1 = reinterpret_cast<unsigned int*>(sm + kSums + 24 * S);
-  t.count = reinterpret_cast<unsigned int*>(sm + kSums + 28 * S);
+  t.sum = reinterpret_cast<double*>(sm);
+  t.nmin = reinterpret_cast<unsigned long long*>(sm + 8 * S);
+  t.max = reinterpret_cast<unsigned long long*>(sm + 16 * S);
+  t.mmhi = reinterpret_cast<unsigned int*>(sm + 24 * S);
+  t.k1 = reinterpret_cast<unsigned int*>(sm + 32 * S);
+  t.count = reinterpret_cast<unsigned int*>(sm + 36 * S);
   return t;
 }
 
@@ -875,12 +852,10 @@ __device__ __forceinline__ SDTab sdtab(unsigned char* sm) {
 __device__ __forceinline__ void sdslot_accum(const SDTab& t, uint32_t j, const SlotRows& g, double v, bool has_v) {
   if (g.rows) {
     atomicAdd(&t.count[j], g.rows);
-    const uint32_t copy = kDenseSumCopies > 1 ? (threadIdx.x & (kDenseSumCopies - 1)) : 0;
-    if (__double_as_longlong(g.sum) != 0) atomicAdd(&t.sum[copy * (kDenseSmemSlots + 1) + j], g.sum);
+    if (__double_as_longlong(g.sum) != 0) atomicAdd(&t.sum[j], g.sum);
   }
   if (!has_v || isnan(v)) return;
   const unsigned long long k = f64_ord_key(v);
-#if FDB_GBD_MMHI
   const unsigned long long w = *reinterpret_cast<volatile unsigned long long*>(&t.mmhi[2 * j]);
   const uint32_t nhi = (uint32_t)(~k >> 32), khi = (uint32_t)(k >> 32);
   const uint32_t nb = (uint32_t)w, kb = (uint32_t)(w >> 32);
@@ -892,10 +867,6 @@ __device__ __forceinline__ void sdslot_accum(const SDTab& t, uint32_t j, const S
     atomicMax(&t.max[j], k);
     if (khi > kb) atomicMax(&t.mmhi[2 * j + 1], khi);
   }
-#else
-  if (~k > *reinterpret_cast<volatile unsigned long long*>(&t.nmin[j])) atomicMax(&t.nmin[j], ~k);
-  if (k > *reinterpret_cast<volatile unsigned long long*>(&t.max[j])) atomicMax(&t.max[j], k);
-#endif
 }
 
 // A value straight into its global slot (no result is used: RED operations).
@@ -911,10 +882,7 @@ __device__ __forceinline__ void dslot_accum(DSlot* d, double v, bool has_v) {
 
 __device__ __forceinline__ void dslot_merge(DSlot* d, const SDTab& t, uint32_t j) {
   atomicAdd(&d->count, (unsigned long long)t.count[j]);
-  double sum = t.sum[j];
-#pragma unroll
-  for (uint32_t c = 1; c < kDenseSumCopies; ++c) sum += t.sum[c * (kDenseSmemSlots + 1) + j];
-  if (__double_as_longlong(sum) != 0) atomicAdd(&d->sum, sum);
+  if (__double_as_longlong(t.sum[j]) != 0) atomicAdd(&d->sum, t.sum[j]);
   if (t.nmin[j]) atomicMax(&d->nmin, t.nmin[j]);
   if (t.max[j]) atomicMax(&d->max, t.max[j]);
 }
@@ -1152,9 +1120,8 @@ __global__ void __launch_bounds__(kDenseCompactThreads)
 // keys that also estimates the groups, and one CTA then aggregates a partition in
 // a shared-memory table that holds all its groups and writes them out: 8 + 16 +
 // 16 + 16 bytes per row, and nothing to clear or compact.  20M rows of 1M keys:
-// split 0.145 ms, aggregation 0.32 (at 81 shared-memory wavefronts per 32 rows and
-// 11 of 32 lanes active: the probes, the SUM's compare-and-swap and MIN / MAX of
-// groups of 20 rows diverge).
+// split 0.144 ms, aggregation 0.254 (the probes, the SUM's compare-and-swap and
+// MIN / MAX of groups of 20 rows diverge).
 struct alignas(16) GbRec {
   uint64_t key;  // as stored (XOR 2^63)
   uint64_t val;  // the value's double bits; kNullVal for NULL
@@ -1514,9 +1481,9 @@ static void launch_dense(Ctx& c, const fdb_dev_column* cols, int nc, uint64_t n,
   switch (nc) {
     case 2:
       if (n < kDenseSmallRows)
-        launch_stream_gb<Op, 2, FDB_GBD_TR / 2, FDB_GBD_ST + 1, FDB_GBD_NCW>(c, cols, n, p, Op::kSmem);
+        launch_stream_gb<Op, 2, kDenseTile / 2, kDenseStages + 1, kDenseWarps>(c, cols, n, p, Op::kSmem);
       else
-        launch_stream_gb<Op, 2, FDB_GBD_TR, FDB_GBD_ST, FDB_GBD_NCW>(c, cols, n, p, Op::kSmem);
+        launch_stream_gb<Op, 2, kDenseTile, kDenseStages, kDenseWarps>(c, cols, n, p, Op::kSmem);
       break;
     // Still two CTAs per SM beside the WHERE columns (40M rows, one column:
     // 800 uniform keys 0.56 ms, 0.74 with tiles of 1024 and one CTA).

@@ -330,8 +330,8 @@ __global__ void __launch_bounds__(256, 8)
           const uint64_t b = pvoff + i;
           if (!pvalid || ((pvalid[b >> 6] >> (b & 63)) & 1ull)) pay = (unsigned long long)payload[i];
         }
-        // The group's sum to its first lane: each lane adds the next one above,
-        // then every other lane drops out.
+        // The group's sum to its first lane, by the method of gtable.cuh's
+        // warp_slot_rows: each lane adds the next one above, then every other drops out.
         unsigned above = peers & ~((2u << lane) - 1u);
         while (__any_sync(0xffffffffu, above != 0)) {
           const unsigned long long x = __shfl_sync(0xffffffffu, pay, above ? __ffs(above) - 1 : (int)lane);

@@ -754,7 +754,7 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
     set((const void*)msd_sample_kernel<Src, kMsdSampleItems>, sizeof(MsdSampleSmem));
     set((const void*)msd_sample_kernel<Src, 2 * kMsdSampleItems>, sizeof(MsdSampleSmem));
     set((const void*)msd_split_kernel<Src, false>, sizeof(MsdSplitSmem));
-    set((const void*)msd_split_kernel<Src, true>, sizeof(MsdSplitSmem));
+    set((const void*)msd_split_kernel<MsdNoSource, true>, sizeof(MsdSplitSmem));
     set((const void*)msd_leaf_kernel<Src, false>, sizeof(MsdLeafSmem<kMsdLeafItems>));
     set((const void*)msd_leaf_kernel<Src, true>, sizeof(MsdLeafSmem<kMsdLeafItems>));
     set((const void*)msd_big_leaf_kernel<Src, false, false>, sizeof(MsdLeafSmem<kMsdBigItems>));
@@ -844,8 +844,8 @@ static bool msd_sort(Ctx& c, const Src& src, uint64_t m64, uint32_t* rows, unsig
       msd_subsample_kernel<8><<<p.parts1, 1024, 0, c.stream>>>(k1, cur1, p.cap1, p.parts2, p.spill, map2, first, state);
     else
       msd_subsample_kernel<16><<<p.parts1, 1024, 0, c.stream>>>(k1, cur1, p.cap1, p.parts2, p.spill, map2, first, state);
-    msd_split_kernel<Src, true><<<tiles + p.parts1, kMsdThreads, sizeof(MsdSplitSmem), c.stream>>>(
-        src, m, k1, v1, cur1, p.cap1, first, p.parts1, map2, p.parts2, p.cap2, k2, v2, cur2, spill, state);
+    msd_split_kernel<MsdNoSource, true><<<tiles + p.parts1, kMsdThreads, sizeof(MsdSplitSmem), c.stream>>>(
+        MsdNoSource{}, m, k1, v1, cur1, p.cap1, first, p.parts1, map2, p.parts2, p.cap2, k2, v2, cur2, spill, state);
     msd_leaves_kernel<<<p.parts1, kMsdThreads, 0, c.stream>>>(cur1, cur2, p.cap2, map2, p.parts2, leaf, big, state);
     lk = k2;
     lv = v2;

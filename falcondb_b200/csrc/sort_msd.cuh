@@ -430,6 +430,16 @@ struct MsdSplitSmem {
   uint32_t scan[32];
 };
 
+// The second level reads the first's pairs, of whatever column.
+struct MsdNoSource {
+  __device__ __forceinline__ uint64_t key(uint32_t) const { return 0; }
+};
+struct MsdSpill {
+  uint64_t* keys;
+  uint32_t* pos;
+  uint32_t cap;
+};
+
 // Pairs of one level scattered into `parts` buckets each.  First level
 // (kSecond false): tile blockIdx.x of the source, buckets 0 .. parts - 1.
 // Second level: the tiles of the first level's buckets (kin, vin, in_count,
@@ -438,12 +448,8 @@ struct MsdSplitSmem {
 // pairs beyond their region go to the spill list.  Bound by
 // shared memory (a table read, one atomic and two or three stores at random
 // places per pair: the LSU data pipe is 72 % busy) and by the write of short
-// runs; 0.68 and 0.84 ms for 100M pairs, 2.9 TB/s.
-struct MsdSpill {
-  uint64_t* keys;
-  uint32_t* pos;
-  uint32_t cap;
-};
+// runs; 0.68 and 0.84 ms for 100M pairs, 2.9 TB/s.  At three CTAs per SM the 40
+// registers do not hold eight keys and eight places: 36 to 88 bytes spill.
 template <class Src, bool kSecond>
 __global__ void __launch_bounds__(kMsdThreads, 3)
     msd_split_kernel(Src src, uint32_t m, const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin,
