@@ -811,8 +811,10 @@ constexpr uint32_t kDenseProbe = FDB_GBD_PROBE;
 constexpr int kDenseTile = 1024, kDenseStages = 2, kDenseWarps = 16;
 // Fewer rows than this leave CTAs without tiles: half as large ones (this kernel, 3000
 // keys: 100,000 rows 18.7 us, 27.5 with whole ones; 600,000 27.3 and 31.6; 1M 40.3 and
-// 35.3).
-constexpr uint64_t kDenseSmallRows = 700'000;
+// 35.3).  So do domains whose rows mostly spill, where the CTAs' tables are no longer
+// what bounds it (100M Zipf rows of 10M values 1.545 ms, 1.552 with whole ones; of 1M
+// the same).
+constexpr uint64_t kDenseSmallRows = 700'000, kDenseWideSlots = 1u << 22;
 // Tiles from one look at whether a warp's rows are worth merging to the next.
 constexpr uint32_t kDenseMergeTiles = 16;
 
@@ -1480,7 +1482,7 @@ static void launch_dense(Ctx& c, const fdb_dev_column* cols, int nc, uint64_t n,
   using Op = GbDenseOp<kDirect>;
   switch (nc) {
     case 2:
-      if (n < kDenseSmallRows)
+      if (n < kDenseSmallRows || p.slots >= kDenseWideSlots)
         launch_stream_gb<Op, 2, kDenseTile / 2, kDenseStages + 1, kDenseWarps>(c, cols, n, p, Op::kSmem);
       else
         launch_stream_gb<Op, 2, kDenseTile, kDenseStages, kDenseWarps>(c, cols, n, p, Op::kSmem);
