@@ -7,8 +7,8 @@
 //
 // Two paths, chosen by a sample of the keys (sort_msd.cuh, msd_sample_kernel):
 // keys that rarely repeat go through the sample sort, the others through the
-// radix passes.  100M float64 keys: 2.6 ms (sample 0.02, first split 0.68,
-// second-level samples 0.11, second split 0.84, leaves 0.81) where the eight
+// radix passes.  100M float64 keys: 2.5 ms (sample 0.04, first split 0.67,
+// second-level samples 0.11, second split 0.78, leaves 0.80) where the eight
 // radix passes take 7.8; 1M: 0.15 against 0.31; DISTINCT over 80M: 2.2 against 7.8.
 //
 // The radix passes: a stable LSD radix sort of (order key, row) pairs with 8-bit digits:

@@ -448,7 +448,7 @@ struct MsdSpill {
 // pairs beyond their region go to the spill list.  Bound by
 // shared memory (a table read, one atomic and two or three stores at random
 // places per pair: the LSU data pipe is 72 % busy) and by the write of short
-// runs; 0.68 and 0.84 ms for 100M pairs, 2.9 TB/s.  At three CTAs per SM the 40
+// runs; 0.67 and 0.78 ms for 100M pairs, 3.0 TB/s.  At three CTAs per SM the 40
 // registers do not hold eight keys and eight places: 36 to 88 bytes spill.
 template <class Src, bool kSecond>
 __global__ void __launch_bounds__(kMsdThreads, 3)
